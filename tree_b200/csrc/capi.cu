@@ -291,7 +291,7 @@ void enqueue_force(tree_gpu_handle* h, bool with_rdf, EventSet* ev) {
   tg::TreeView tv = tree_view(h);
   tg::WalkParams wp = walk_params(h);
   if (h->prm.precision == TREE_GPU_PREC_FP64) {
-    tg::walk64(h->x, h->n, (int)h->n_el, h->b.vals, tv, wp, h->f,
+    tg::walk64(h->x, h->n, (int)h->n_el, h->b.vals, tv, h->b.mx.kids, wp, h->f,
                h->epot_part, with_rdf ? h->rdf : nullptr, h->counters,
                h->b.err, st);
     h->timing.launches += h->n > 0 ? 1 : 0;

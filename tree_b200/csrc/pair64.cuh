@@ -1,5 +1,8 @@
 // pair64.cuh -- FP64 leaf pair laws shared by the parity walk and the direct
-// sum (both compiled -fmad=false).  Operation order follows tree.f90.
+// sum (both compiled -fmad=false).  leaf_pair64 follows tree.f90's operation
+// order; pairs far enough apart that their law is plain Coulomb to double
+// precision -- nearly all of them -- take pair64_coulomb, one reciprocal
+// square root instead of a square root and four to six IEEE divisions.
 #pragma once
 #include "internal.cuh"
 #include "walk.h"
@@ -78,6 +81,31 @@ __device__ __forceinline__ bool leaf_pair64(double xr0, double xr1, double xr2,
   f2 = f2 + fr * xr2;
   r_out = r;
   return true;
+}
+
+// Squared distance beyond which leaf_pair64's law equals q q' eps / r to
+// double precision: for REF same-species pairs the cutoff itself (closer ones
+// contribute nothing); for REF e-i pairs r > 45 rs, where exp(-r/rs) (1 + r/rs)
+// < 2e-18; for KELBG x^2 > 40 (with a margin for its rounding), the point
+// where leaf_pair64 drops the exponential too.
+template <int PHYS>
+__device__ __forceinline__ double pair64_far2(bool same, int tsp, const WalkParams& wp) {
+  if (PHYS == 0) return same ? 0.01 : 2025.0 * (wp.rs * wp.rs);
+  const double lam = same ? (tsp == 0 ? wp.lam_ee : wp.lam_ii) : wp.lam_ei;
+  return 40.001 * (lam * lam);
+}
+
+// Adds a plain Coulomb pair; q = +eps for like charges, -eps for unlike ones.
+__device__ __forceinline__ void pair64_coulomb(double xr0, double xr1, double xr2, double r2,
+                                               double q, double& f0, double& f1, double& f2,
+                                               double& ep) {
+  const double rinv = rsqrt(r2);
+  const double ph = q * rinv;
+  const double fr = ph * (rinv * rinv);
+  ep = __fma_rn(0.5, ph, ep);
+  f0 = __fma_rn(fr, xr0, f0);
+  f1 = __fma_rn(fr, xr1, f1);
+  f2 = __fma_rn(fr, xr2, f2);
 }
 
 }  // namespace tg

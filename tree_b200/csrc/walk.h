@@ -15,9 +15,10 @@ struct WalkParams {
 };
 
 // FP64 per-target walk (parity path).  rdf may be null (2 x 10001 u32).
-// counters[0] += accepted cells, counters[1] += leaf pairs.
+// counters[0] += accepted cells, counters[1] += leaf pairs.  kids: the child
+// table of both trees, 8 per node (-1: none), every child after its parent.
 void walk64(const double* x, int n, int n_el, const uint32_t* order,
-            const TreeView& tv, const WalkParams& wp, double* f,
+            const TreeView& tv, const int32_t* kids, const WalkParams& wp, double* f,
             double2* epot_part, uint32_t* rdf, unsigned long long* counters,
             int32_t* err, cudaStream_t st);
 
