@@ -190,7 +190,8 @@ int tree_gpu_get_state(tree_gpu_handle* h, double* x_el, double* v_el,
  * pair laws and no tree (the theta -> 0 limit of Search_Tree_*,
  * tree.f90:721-1133).  targets: global indices (electrons 0..n_el-1, ions
  * n_el..n_el+n_ion-1).  Out (host): f (3*nt), epot (nt; 0.5*sum of V per
- * target).  Allocates its device scratch per call. */
+ * target).  Its device scratch (about 32 bytes per target and source chunk)
+ * stays with the handle and grows to the largest call. */
 int tree_gpu_direct(tree_gpu_handle* h, const int64_t* targets, int64_t nt,
                     double* f, double* epot);
 

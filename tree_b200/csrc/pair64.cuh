@@ -1,8 +1,7 @@
 // pair64.cuh -- FP64 leaf pair laws shared by the parity walk and the direct
 // sum (both compiled -fmad=false).  leaf_pair64 follows tree.f90's operation
 // order; pairs far enough apart that their law is plain Coulomb to double
-// precision -- nearly all of them -- take pair64_coulomb, one reciprocal
-// square root instead of a square root and four to six IEEE divisions.
+// precision (pair64_far2) -- nearly all of them -- take shorter forms.
 #pragma once
 #include "internal.cuh"
 #include "walk.h"
@@ -93,19 +92,6 @@ __device__ __forceinline__ double pair64_far2(bool same, int tsp, const WalkPara
   if (PHYS == 0) return same ? 0.01 : 2025.0 * (wp.rs * wp.rs);
   const double lam = same ? (tsp == 0 ? wp.lam_ee : wp.lam_ii) : wp.lam_ei;
   return 40.001 * (lam * lam);
-}
-
-// Adds a plain Coulomb pair; q = +eps for like charges, -eps for unlike ones.
-__device__ __forceinline__ void pair64_coulomb(double xr0, double xr1, double xr2, double r2,
-                                               double q, double& f0, double& f1, double& f2,
-                                               double& ep) {
-  const double rinv = rsqrt(r2);
-  const double ph = q * rinv;
-  const double fr = ph * (rinv * rinv);
-  ep = __fma_rn(0.5, ph, ep);
-  f0 = __fma_rn(fr, xr0, f0);
-  f1 = __fma_rn(fr, xr1, f1);
-  f2 = __fma_rn(fr, xr2, f2);
 }
 
 }  // namespace tg
