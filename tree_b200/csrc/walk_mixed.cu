@@ -197,137 +197,141 @@ __device__ __forceinline__ double warp_max_d(double v) {
 }
 
 // ---------------------------------------------------------------- M2P ----
-// Net monopole Q, dipole D, trace-free second moment S (from 1/2 sum q a a^T)
-// and, for ORDER 3, trace-free third moment T (from sum q a a a) about the
-// cell centroid.  With d = target - centroid, r = |d|:
-//   phi = Q/r + D.d/r^3 + 3 d.S.d/r^5 + 5/2 T(d,d,d)/r^7
-//   -grad phi = g d - D/r^3 - 6 S d/r^5 - 7.5 T(.,d,d)/r^7,
-//   g = Q/r^3 + 3 D.d/r^5 + 15 d.S.d/r^7 + 17.5 T(d,d,d)/r^9.
-// About 50 flop per entry at ORDER 2, 100 at ORDER 3 (FMA = 2).  The ion part
+// Net monopole Q, dipole D, trace-free second moment S (from 1/2 sum q a a^T),
+// third moment T (from sum q a a a) and fourth moment H about the cell
+// centroid.  With d = target - centroid, r = |d|, s = 1/r, n = d / r:
+//   phi = s [Q + s (D.n + s (S'nn + s (T'nnn + s H'nnnn)))],
+//   -grad phi = s^2 (g n - s W),  g = r phi + 2 s n.W,
+//   W = D + 2 s (S'n + 3/2 s (T'nn + 4/3 s H'nnn)),
+// with S' = 3 S, T' = 5/2 T, H' = 35/8 H: the prefactors of each order are
+// taken into the moments when a cell is staged (once per 32 targets), and the
+// force needs no scalar of its own beyond n.W.  Normalised form: every
+// intermediate is bounded by n (a/r)^k -- escaped electrons millions of um
+// away would otherwise overflow T(d,d,d) ~ |T| r^3 while 1/r^7 underflows.
+// T is trace-free (T_iik = 0), so T_kzz = -T_kxx - T_kyy and each component
+// of T(., n, n) takes five terms with a2 = nx^2 - nz^2, b2 = ny^2 - nz^2; each
+// component of H(., n, n, n) is a combination of seven cubic harmonics P1..P7
+// of n, its z component reading the dependent components xxzz, xyzz, yyzz
+// staged with the others.  About 105 multiply-adds at order 4.  The ion part
 // of phi for the Epot_e/Epot_i split is taken at monopole order (q_ion / r).
+
+// 1/sqrt(x) of a normal number, without rsqrtf's rescaling of subnormal ones.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The rows of a staged cell (WarpSmem::cell), moments scaled as above.
+template <int ORDER, int ROWS>
+__device__ __forceinline__ void m2p_rows(const MixedArgs& a, int node, double Gx, double Gy,
+                                         double Gz, float4 (&r)[ROWS]) {
+  const double4 c = ldg_d4(&a.node_c[node]);
+  const float4* mp = a.mom + 3 * (int64_t)node;
+  const float4 m0 = __ldg(mp), m1 = __ldg(mp + 1), m2 = __ldg(mp + 2);
+  r[0] = make_float4((float)(Gx - c.x), (float)(Gy - c.y), (float)(Gz - c.z), m0.x);
+  r[1] = make_float4(m0.y, m0.z, m0.w, m2.w);
+  r[2] = make_float4(3.f * m1.x, 3.f * m1.y, 3.f * m1.z, 3.f * m1.w);
+  r[3] = make_float4(3.f * m2.x, 3.f * m2.y, 0.f, 0.f);
+  if constexpr (ORDER >= 3) {
+    const float4* tp = a.mom3 + 3 * (int64_t)node;
+    const float4 t0 = __ldg(tp), t1 = __ldg(tp + 1), t2 = __ldg(tp + 2);
+    r[3].z = 2.5f * t0.x;
+    r[3].w = 2.5f * t0.y;
+    r[4] = make_float4(0.f, 2.5f * t0.w, 2.5f * t1.x, 2.5f * t1.y);
+    r[5] = make_float4(2.5f * t1.z, 2.5f * t1.w, 2.5f * t2.x, 2.5f * t2.y);
+  }
+  if constexpr (ORDER >= 4) {
+    const float4* hp = a.mom4 + 3 * (int64_t)node;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float4 h = __ldg(hp + k);
+      r[6 + k] = make_float4(4.375f * h.x, 4.375f * h.y, 4.375f * h.z, 4.375f * h.w);
+    }
+  }
+}
+
 template <int ORDER>
 __device__ __forceinline__ void eval_m2p(WarpSmem& sm, int head, int cnt,
                                          const MixedArgs& a, double Gx,
                                          double Gy, double Gz, float tx,
                                          float ty, float tz, int lane,
                                          Acc& acc) {
+  constexpr int kRows = ORDER >= 4 ? 9 : (ORDER == 3 ? 6 : 4);
   if (lane < cnt) {
-    int node = sm.m2p[(head + lane) & (kM2pRing - 1)];
-    double4 c = ldg_d4(&a.node_c[node]);
-    const float4* mp = a.mom + 3 * (int64_t)node;
-    float4 m0 = __ldg(mp), m1 = __ldg(mp + 1), m2 = __ldg(mp + 2);
+    float4 r[kRows];
+    m2p_rows<ORDER>(a, sm.m2p[(head + lane) & (kM2pRing - 1)], Gx, Gy, Gz, r);
     float4* cl = sm.cell + kCellF4 * lane;
-    cl[0] = make_float4((float)(c.x - Gx), (float)(c.y - Gy), (float)(c.z - Gz), m0.x);
-    cl[1] = make_float4(m0.y, m0.z, m0.w, m2.w);
-    cl[2] = m1;
-    if (ORDER >= 3) {
-      const float4* tp = a.mom3 + 3 * (int64_t)node;
-      const float4 t0 = __ldg(tp), t1 = __ldg(tp + 1), t2 = __ldg(tp + 2);
-      cl[3] = make_float4(m2.x, m2.y, t0.x, t0.y);
-      cl[4] = make_float4(t0.z, t0.w, t1.x, t1.y);
-      cl[5] = make_float4(t1.z, t1.w, t2.x, t2.y);
-    } else {
-      cl[3] = make_float4(m2.x, m2.y, 0.f, 0.f);
-    }
-    if (ORDER >= 4) {
-      const float4* hp = a.mom4 + 3 * (int64_t)node;
-      cl[6] = __ldg(hp);
-      cl[7] = __ldg(hp + 1);
-      cl[8] = __ldg(hp + 2);
-    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) cl[j] = r[j];
   }
   __syncwarp();
   float fx = 0.f, fy = 0.f, fz = 0.f, pa = 0.f, pi = 0.f;
 #pragma unroll 1
   for (int k = 0; k < cnt; ++k) {
     const float4* cl = sm.cell + kCellF4 * k;
-    const float4 A = cl[0], B = cl[1], C = cl[2], E = cl[3];
-    const float dx = tx - A.x, dy = ty - A.y, dz = tz - A.z;
+    const float4 A = cl[0];
+    const float dx = tx + A.x, dy = ty + A.y, dz = tz + A.z;
     // accepted cells are farther than rcrit >= 0; the 1e-30 only guards a
     // zero-size cell against an FP32 distance of 0
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 1e-30f)));
-    // Normalised form: the moments are contracted with the unit vector
-    // n = d / r and scaled by powers of s = 1/r, so every intermediate is
-    // bounded by n (a/r)^k -- escaped electrons millions of um away would
-    // otherwise overflow T(d,d,d) ~ |T| r^3 while 1/r^7 underflows.
-    const float s = rsqrtf(r2), s2 = s * s;
+    const float s = rsqrt_normal(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 1e-30f))));
     const float nx = dx * s, ny = dy * s, nz = dz * s;
-    // S n with S = [[Sxx,Sxy,Szx],[Sxy,Syy,Syz],[Szx,Syz,Szz]]
-    const float Sx = fmaf(C.x, nx, fmaf(C.w, ny, E.y * nz));
-    const float Sy = fmaf(C.w, nx, fmaf(C.y, ny, E.x * nz));
-    const float Sz = fmaf(E.y, nx, fmaf(E.x, ny, C.z * nz));
-    const float u = fmaf(nx, Sx, fmaf(ny, Sy, nz * Sz));
-    const float Dn = fmaf(B.x, nx, fmaf(B.y, ny, B.z * nz));
-    // r^2 (-grad phi) = gp n - s D - 6 s^2 S n - 7.5 s^3 T(., n, n),
-    // gp = Q + 3 s D.n + 15 s^2 n.S.n + 17.5 s^3 T(n,n,n);
-    // r phi = Q + s D.n + 3 s^2 n.S.n + 2.5 s^3 T(n,n,n)
-    const float su = s * u;
-    float gp = fmaf(s, fmaf(15.f, su, 3.f * Dn), A.w);
-    float php = fmaf(s, fmaf(3.f, su, Dn), A.w);
-    const float c5 = -6.f * s2;
-    float gx = fmaf(c5, Sx, -s * B.x);
-    float gy = fmaf(c5, Sy, -s * B.y);
-    float gz = fmaf(c5, Sz, -s * B.z);
+    const float xx = nx * nx, yy = ny * ny, zz = nz * nz;
+    const float a2 = xx - zz, b2 = yy - zz;
+    float Wx = 0.f, Wy = 0.f, Wz = 0.f, ph = 0.f, w = 0.f;
+    const float4 E = cl[3];
+    if (ORDER >= 4) {
+      const float4 H0 = cl[6], H1 = cl[7], H2 = cl[8];
+      const float x3 = 3.f * nx, y3 = 3.f * ny;
+      const float P1 = nx * fmaf(-3.f, zz, xx), P6 = ny * fmaf(-3.f, zz, yy);
+      const float P2 = y3 * a2, P4 = x3 * b2;
+      const float P3 = nz * fmaf(3.f, xx, -zz), P7 = nz * fmaf(3.f, yy, -zz);
+      const float P5 = x3 * (2.f * ny * nz);
+      // (xxxx xxxy xxxz xxyy) (xxyz xyyy xyyz yyyy) (yyyz xxzz xyzz yyzz)
+      Wx = fmaf(H0.x, P1, fmaf(H0.y, P2, fmaf(H0.z, P3, fmaf(H0.w, P4,
+           fmaf(H1.x, P5, fmaf(H1.y, P6, H1.z * P7))))));
+      Wy = fmaf(H0.y, P1, fmaf(H0.w, P2, fmaf(H1.x, P3, fmaf(H1.y, P4,
+           fmaf(H1.z, P5, fmaf(H1.w, P6, H2.x * P7))))));
+      Wz = fmaf(H0.z, P1, fmaf(H1.x, P2, fmaf(H2.y, P3, fmaf(H1.z, P4,
+           fmaf(H2.z, P5, fmaf(H2.x, P6, H2.w * P7))))));
+      ph = fmaf(nx, Wx, fmaf(ny, Wy, nz * Wz));
+      w = ph;
+    }
     if (ORDER >= 3) {
+      // xxx = E.z, yyy = E.w, xxy = T1.y, xxz = T1.z, xyy = T1.w, yyz = T2.x,
+      // xzz = T2.y, yzz = T2.z, xyz = T2.w
       const float4 T1 = cl[4], T2 = cl[5];
-      // T order: xxx = E.z, yyy = E.w, zzz = T1.x, xxy = T1.y, xxz = T1.z,
-      // xyy = T1.w, yyz = T2.x, xzz = T2.y, yzz = T2.z, xyz = T2.w.  T is
-      // trace-free (T_iik = 0), so T_kzz = -T_kxx - T_kyy and each component
-      // of T(., n, n) takes five terms with a = nx^2 - nz^2, b = ny^2 - nz^2
-      const float zz = nz * nz;
-      const float a2 = fmaf(nx, nx, -zz), b2 = fmaf(ny, ny, -zz);
       const float x2 = nx + nx, y2 = ny + ny;
       const float xy2 = x2 * ny, xz2 = x2 * nz, yz2 = y2 * nz;
       const float Tx = fmaf(E.z, a2, fmaf(T1.w, b2, fmaf(T1.y, xy2, fmaf(T1.z, xz2, T2.w * yz2))));
       const float Ty = fmaf(T1.y, a2, fmaf(E.w, b2, fmaf(T1.w, xy2, fmaf(T2.w, xz2, T2.x * yz2))));
       const float Tz = fmaf(T1.z, a2, fmaf(T2.x, b2, fmaf(T2.w, xy2, fmaf(T2.y, xz2, T2.z * yz2))));
-      const float T3 = fmaf(nx, Tx, fmaf(ny, Ty, nz * Tz));
-      const float s3 = s2 * s;
-      const float s3T3 = s3 * T3;
-      gp = fmaf(17.5f, s3T3, gp);
-      php = fmaf(2.5f, s3T3, php);
-      const float c7 = -7.5f * s3;
-      gx = fmaf(c7, Tx, gx);
-      gy = fmaf(c7, Ty, gy);
-      gz = fmaf(c7, Tz, gz);
+      const float t = fmaf(nx, Tx, fmaf(ny, Ty, nz * Tz));
+      const float s43 = (4.f / 3.f) * s;
+      Wx = fmaf(s43, Wx, Tx);
+      Wy = fmaf(s43, Wy, Ty);
+      Wz = fmaf(s43, Wz, Tz);
+      ph = fmaf(s, ph, t);
+      w = fmaf(s43, w, t);
     }
-    if (ORDER >= 4) {
-      // hexadecapole: r^2 (-grad phi) += 39.375 s^4 H(n,n,n,n) n - 17.5 s^4
-      // H(., n, n, n); r phi += 4.375 s^4 H(n,n,n,n) (phi = 35/8 H(d,d,d,d)
-      // / r^9).  H is trace-free, so each component of H(., n, n, n) is a
-      // combination of seven cubic harmonics P1..P7 of n; the z component
-      // reads the three dependent components xxzz, xyzz, yyzz staged with
-      // the others.
-      const float4 H0 = cl[6], H1 = cl[7], H2 = cl[8];
-      const float xx = nx * nx, yy = ny * ny, zz3 = 3.f * nz * nz;
-      const float P1 = nx * (xx - zz3);
-      const float P6 = ny * (yy - zz3);
-      const float P2 = 3.f * ny * fmaf(nz, -nz, xx);
-      const float P4 = 3.f * nx * fmaf(nz, -nz, yy);
-      const float P3 = nz * fmaf(3.f, xx, -nz * nz);
-      const float P7 = nz * fmaf(3.f, yy, -nz * nz);
-      const float P5 = 6.f * nx * ny * nz;
-      // (xxxx xxxy xxxz xxyy) (xxyz xyyy xyyz yyyy) (yyyz xxzz xyzz yyzz)
-      const float Vx = fmaf(H0.x, P1, fmaf(H0.y, P2, fmaf(H0.z, P3, fmaf(H0.w, P4,
-                       fmaf(H1.x, P5, fmaf(H1.y, P6, H1.z * P7))))));
-      const float Vy = fmaf(H0.y, P1, fmaf(H0.w, P2, fmaf(H1.x, P3, fmaf(H1.y, P4,
-                       fmaf(H1.z, P5, fmaf(H1.w, P6, H2.x * P7))))));
-      const float Vz = fmaf(H0.z, P1, fmaf(H1.x, P2, fmaf(H2.y, P3, fmaf(H1.z, P4,
-                       fmaf(H2.z, P5, fmaf(H2.x, P6, H2.w * P7))))));
-      const float H4 = fmaf(nx, Vx, fmaf(ny, Vy, nz * Vz));
-      const float s4 = s2 * s2;
-      const float s4H = s4 * H4;
-      gp = fmaf(39.375f, s4H, gp);
-      php = fmaf(4.375f, s4H, php);
-      const float c9 = -17.5f * s4;
-      gx = fmaf(c9, Vx, gx);
-      gy = fmaf(c9, Vy, gy);
-      gz = fmaf(c9, Vz, gz);
-    }
-    fx = fmaf(s2, fmaf(gp, nx, gx), fx);
-    fy = fmaf(s2, fmaf(gp, ny, gy), fy);
-    fz = fmaf(s2, fmaf(gp, nz, gz), fz);
-    pa = fmaf(s, php, pa);
+    const float4 B = cl[1], C = cl[2];
+    // S n with S = [[Sxx,Sxy,Szx],[Sxy,Syy,Syz],[Szx,Syz,Szz]]
+    const float Sx = fmaf(C.x, nx, fmaf(C.w, ny, E.y * nz));
+    const float Sy = fmaf(C.w, nx, fmaf(C.y, ny, E.x * nz));
+    const float Sz = fmaf(E.y, nx, fmaf(E.x, ny, C.z * nz));
+    const float u = fmaf(nx, Sx, fmaf(ny, Sy, nz * Sz));
+    const float s15 = 1.5f * s, s2x = s + s;
+    Wx = fmaf(s2x, fmaf(s15, Wx, Sx), B.x);
+    Wy = fmaf(s2x, fmaf(s15, Wy, Sy), B.y);
+    Wz = fmaf(s2x, fmaf(s15, Wz, Sz), B.z);
+    const float Dn = fmaf(B.x, nx, fmaf(B.y, ny, B.z * nz));
+    ph = fmaf(s, fmaf(s, fmaf(s, ph, u), Dn), A.w);
+    w = fmaf(s2x, fmaf(s15, w, u), Dn);
+    const float s2 = s * s, g = s2 * fmaf(s2x, w, ph), ms3 = -s * s2;
+    fx = fmaf(g, nx, fmaf(ms3, Wx, fx));
+    fy = fmaf(g, ny, fmaf(ms3, Wy, fy));
+    fz = fmaf(g, nz, fmaf(ms3, Wz, fz));
+    pa = fmaf(s, ph, pa);
     pi = fmaf(B.w, s, pi);
   }
   __syncwarp();
@@ -358,28 +362,7 @@ __device__ __forceinline__ void eval_m2p_x2(WarpSmem& sm, int head, int cnt,
     // chargeless dummy far away past cnt
     float4 r[kRows];
     if (lane < cnt) {
-      const int node = sm.m2p[(head + lane) & (kM2pRing - 1)];
-      const double4 c = ldg_d4(&a.node_c[node]);
-      const float4* mp = a.mom + 3 * (int64_t)node;
-      const float4 m0 = __ldg(mp), m1 = __ldg(mp + 1), m2 = __ldg(mp + 2);
-      r[0] = make_float4((float)(c.x - Gx), (float)(c.y - Gy), (float)(c.z - Gz), m0.x);
-      r[1] = make_float4(m0.y, m0.z, m0.w, m2.w);
-      r[2] = m1;
-      if (ORDER >= 3) {
-        const float4* tp = a.mom3 + 3 * (int64_t)node;
-        const float4 t0 = __ldg(tp), t1 = __ldg(tp + 1), t2 = __ldg(tp + 2);
-        r[3] = make_float4(m2.x, m2.y, t0.x, t0.y);
-        r[4] = make_float4(t0.z, t0.w, t1.x, t1.y);
-        r[5] = make_float4(t1.z, t1.w, t2.x, t2.y);
-      } else {
-        r[3] = make_float4(m2.x, m2.y, 0.f, 0.f);
-      }
-      if (ORDER >= 4) {
-        const float4* hp = a.mom4 + 3 * (int64_t)node;
-        r[6] = __ldg(hp);
-        r[7] = __ldg(hp + 1);
-        r[8] = __ldg(hp + 2);
-      }
+      m2p_rows<ORDER>(a, sm.m2p[(head + lane) & (kM2pRing - 1)], Gx, Gy, Gz, r);
     } else {
       r[0] = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f);
 #pragma unroll
@@ -409,65 +392,15 @@ __device__ __forceinline__ void eval_m2p_x2(WarpSmem& sm, int head, int cnt,
     const float2 Ax = make_float2(q.x, q.y), Ay = make_float2(q.z, q.w);
     q = bl[1];
     const float2 Az = make_float2(q.x, q.y), Q = make_float2(q.z, q.w);
-    q = bl[2];
-    const float2 Dx = make_float2(q.x, q.y), Dy = make_float2(q.z, q.w);
-    q = bl[3];
-    const float2 Dz = make_float2(q.x, q.y), Qi = make_float2(q.z, q.w);
-    q = bl[4];
-    const float2 Sxx = make_float2(q.x, q.y), Syy = make_float2(q.z, q.w);
-    q = bl[5];
-    const float2 Szz = make_float2(q.x, q.y), Sxy = make_float2(q.z, q.w);
-    q = bl[6];
-    const float2 Syz = make_float2(q.x, q.y), Szx = make_float2(q.z, q.w);
-    const float2 dx = add2(tx2, make_float2(-Ax.x, -Ax.y));
-    const float2 dy = add2(ty2, make_float2(-Ay.x, -Ay.y));
-    const float2 dz = add2(tz2, make_float2(-Az.x, -Az.y));
+    const float2 dx = add2(tx2, Ax), dy = add2(ty2, Ay), dz = add2(tz2, Az);
     const float2 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, f2(1e-30f))));
-    const float2 s = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-    const float2 s2 = mul2(s, s);
+    const float2 s = make_float2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
     const float2 nx = mul2(dx, s), ny = mul2(dy, s), nz = mul2(dz, s);
-    const float2 Sx = fma2(Sxx, nx, fma2(Sxy, ny, mul2(Szx, nz)));
-    const float2 Sy = fma2(Sxy, nx, fma2(Syy, ny, mul2(Syz, nz)));
-    const float2 Sz = fma2(Szx, nx, fma2(Syz, ny, mul2(Szz, nz)));
-    const float2 u = fma2(nx, Sx, fma2(ny, Sy, mul2(nz, Sz)));
-    const float2 Dn = fma2(Dx, nx, fma2(Dy, ny, mul2(Dz, nz)));
-    const float2 su = mul2(s, u);
-    float2 gp = fma2(s, fma2(f2(15.f), su, mul2(f2(3.f), Dn)), Q);
-    float2 php = fma2(s, fma2(f2(3.f), su, Dn), Q);
-    const float2 c5 = mul2(f2(-6.f), s2);
-    const float2 ms = make_float2(-s.x, -s.y);
-    float2 gx = fma2(c5, Sx, mul2(ms, Dx));
-    float2 gy = fma2(c5, Sy, mul2(ms, Dy));
-    float2 gz = fma2(c5, Sz, mul2(ms, Dz));
-    if (ORDER >= 3) {
-      // (Syz Szx Txxx Tyyy) (Tzzz Txxy Txxz Txyy) (Tyyz Txzz Tyzz Txyz)
-      q = bl[7];
-      const float2 Txxx = make_float2(q.x, q.y), Tyyy = make_float2(q.z, q.w);
-      q = bl[8];
-      const float2 Txxy = make_float2(q.z, q.w);
-      q = bl[9];
-      const float2 Txxz = make_float2(q.x, q.y), Txyy = make_float2(q.z, q.w);
-      q = bl[10];
-      const float2 Tyyz = make_float2(q.x, q.y), Txzz = make_float2(q.z, q.w);
-      q = bl[11];
-      const float2 Tyzz = make_float2(q.x, q.y), Txyz = make_float2(q.z, q.w);
-      const float2 zz = mul2(nz, nz);
-      const float2 mzz = make_float2(-zz.x, -zz.y);
-      const float2 a2 = fma2(nx, nx, mzz), b2 = fma2(ny, ny, mzz);
-      const float2 x2 = add2(nx, nx), y2 = add2(ny, ny);
-      const float2 xy2 = mul2(x2, ny), xz2 = mul2(x2, nz), yz2 = mul2(y2, nz);
-      const float2 Tx = fma2(Txxx, a2, fma2(Txyy, b2, fma2(Txxy, xy2, fma2(Txxz, xz2, mul2(Txyz, yz2)))));
-      const float2 Ty = fma2(Txxy, a2, fma2(Tyyy, b2, fma2(Txyy, xy2, fma2(Txyz, xz2, mul2(Tyyz, yz2)))));
-      const float2 Tz = fma2(Txxz, a2, fma2(Tyyz, b2, fma2(Txyz, xy2, fma2(Txzz, xz2, mul2(Tyzz, yz2)))));
-      const float2 T3 = fma2(nx, Tx, fma2(ny, Ty, mul2(nz, Tz)));
-      const float2 s3T3 = mul2(mul2(s2, s), T3);
-      gp = fma2(f2(17.5f), s3T3, gp);
-      php = fma2(f2(2.5f), s3T3, php);
-      const float2 c7 = mul2(f2(-7.5f), mul2(s2, s));
-      gx = fma2(c7, Tx, gx);
-      gy = fma2(c7, Ty, gy);
-      gz = fma2(c7, Tz, gz);
-    }
+    const float2 xx = mul2(nx, nx), yy = mul2(ny, ny);
+    const float2 mzz = mul2(nz, mul2(f2(-1.f), nz));
+    const float2 a2 = add2(xx, mzz), b2 = add2(yy, mzz);
+    const float2 yz2 = mul2(add2(ny, ny), nz);
+    float2 Wx = f2(0.f), Wy = Wx, Wz = Wx, ph = Wx, w = Wx;
     if (ORDER >= 4) {
       // (xxxx xxxy xxxz xxyy) (xxyz xyyy xyyz yyyy) (yyyz xxzz xyzz yyzz)
       q = bl[12];
@@ -482,36 +415,74 @@ __device__ __forceinline__ void eval_m2p_x2(WarpSmem& sm, int head, int cnt,
       const float2 H8 = make_float2(q.x, q.y), H9 = make_float2(q.z, q.w);
       q = bl[17];
       const float2 H10 = make_float2(q.x, q.y), H11 = make_float2(q.z, q.w);
-      const float2 xx = mul2(nx, nx), yy = mul2(ny, ny);
-      const float2 zz3 = mul2(f2(3.f), mul2(nz, nz));
-      const float2 mnz = make_float2(-nz.x, -nz.y);
-      const float2 P1 = mul2(nx, add2(xx, make_float2(-zz3.x, -zz3.y)));
-      const float2 P6 = mul2(ny, add2(yy, make_float2(-zz3.x, -zz3.y)));
-      const float2 P2 = mul2(mul2(f2(3.f), ny), fma2(nz, mnz, xx));
-      const float2 P4 = mul2(mul2(f2(3.f), nx), fma2(nz, mnz, yy));
-      const float2 P3 = mul2(nz, fma2(f2(3.f), xx, mul2(mnz, nz)));
-      const float2 P7 = mul2(nz, fma2(f2(3.f), yy, mul2(mnz, nz)));
-      const float2 P5 = mul2(mul2(f2(6.f), nx), mul2(ny, nz));
-      const float2 Vx = fma2(H0, P1, fma2(H1, P2, fma2(H2, P3, fma2(H3, P4,
-                        fma2(H4, P5, fma2(H5, P6, mul2(H6, P7)))))));
-      const float2 Vy = fma2(H1, P1, fma2(H3, P2, fma2(H4, P3, fma2(H5, P4,
-                        fma2(H6, P5, fma2(H7, P6, mul2(H8, P7)))))));
-      const float2 Vz = fma2(H2, P1, fma2(H4, P2, fma2(H9, P3, fma2(H6, P4,
-                        fma2(H10, P5, fma2(H8, P6, mul2(H11, P7)))))));
-      const float2 H4n = fma2(nx, Vx, fma2(ny, Vy, mul2(nz, Vz)));
-      const float2 s4 = mul2(s2, s2);
-      const float2 s4H = mul2(s4, H4n);
-      gp = fma2(f2(39.375f), s4H, gp);
-      php = fma2(f2(4.375f), s4H, php);
-      const float2 c9 = mul2(f2(-17.5f), s4);
-      gx = fma2(c9, Vx, gx);
-      gy = fma2(c9, Vy, gy);
-      gz = fma2(c9, Vz, gz);
+      const float2 x3 = mul2(f2(3.f), nx), y3 = mul2(f2(3.f), ny);
+      const float2 P1 = mul2(nx, fma2(f2(3.f), mzz, xx));
+      const float2 P6 = mul2(ny, fma2(f2(3.f), mzz, yy));
+      const float2 P2 = mul2(y3, a2), P4 = mul2(x3, b2), P5 = mul2(x3, yz2);
+      const float2 P3 = mul2(nz, fma2(f2(3.f), xx, mzz));
+      const float2 P7 = mul2(nz, fma2(f2(3.f), yy, mzz));
+      Wx = fma2(H0, P1, fma2(H1, P2, fma2(H2, P3, fma2(H3, P4,
+           fma2(H4, P5, fma2(H5, P6, mul2(H6, P7)))))));
+      Wy = fma2(H1, P1, fma2(H3, P2, fma2(H4, P3, fma2(H5, P4,
+           fma2(H6, P5, fma2(H7, P6, mul2(H8, P7)))))));
+      Wz = fma2(H2, P1, fma2(H4, P2, fma2(H9, P3, fma2(H6, P4,
+           fma2(H10, P5, fma2(H8, P6, mul2(H11, P7)))))));
+      ph = fma2(nx, Wx, fma2(ny, Wy, mul2(nz, Wz)));
+      w = ph;
     }
-    fx = fma2(s2, fma2(gp, nx, gx), fx);
-    fy = fma2(s2, fma2(gp, ny, gy), fy);
-    fz = fma2(s2, fma2(gp, nz, gz), fz);
-    pa = fma2(s, php, pa);
+    q = bl[6];
+    const float2 Syz = make_float2(q.x, q.y), Szx = make_float2(q.z, q.w);
+    if (ORDER >= 3) {
+      // (Syz Szx Txxx Tyyy) (- Txxy Txxz Txyy) (Tyyz Txzz Tyzz Txyz)
+      q = bl[7];
+      const float2 Txxx = make_float2(q.x, q.y), Tyyy = make_float2(q.z, q.w);
+      q = bl[8];
+      const float2 Txxy = make_float2(q.z, q.w);
+      q = bl[9];
+      const float2 Txxz = make_float2(q.x, q.y), Txyy = make_float2(q.z, q.w);
+      q = bl[10];
+      const float2 Tyyz = make_float2(q.x, q.y), Txzz = make_float2(q.z, q.w);
+      q = bl[11];
+      const float2 Tyzz = make_float2(q.x, q.y), Txyz = make_float2(q.z, q.w);
+      const float2 x2 = add2(nx, nx);
+      const float2 xy2 = mul2(x2, ny), xz2 = mul2(x2, nz);
+      const float2 Tx = fma2(Txxx, a2, fma2(Txyy, b2, fma2(Txxy, xy2, fma2(Txxz, xz2, mul2(Txyz, yz2)))));
+      const float2 Ty = fma2(Txxy, a2, fma2(Tyyy, b2, fma2(Txyy, xy2, fma2(Txyz, xz2, mul2(Tyyz, yz2)))));
+      const float2 Tz = fma2(Txxz, a2, fma2(Tyyz, b2, fma2(Txyz, xy2, fma2(Txzz, xz2, mul2(Tyzz, yz2)))));
+      const float2 t = fma2(nx, Tx, fma2(ny, Ty, mul2(nz, Tz)));
+      const float2 s43 = mul2(f2(4.f / 3.f), s);
+      Wx = fma2(s43, Wx, Tx);
+      Wy = fma2(s43, Wy, Ty);
+      Wz = fma2(s43, Wz, Tz);
+      ph = fma2(s, ph, t);
+      w = fma2(s43, w, t);
+    }
+    q = bl[4];
+    const float2 Sxx = make_float2(q.x, q.y), Syy = make_float2(q.z, q.w);
+    q = bl[5];
+    const float2 Szz = make_float2(q.x, q.y), Sxy = make_float2(q.z, q.w);
+    const float2 Sx = fma2(Sxx, nx, fma2(Sxy, ny, mul2(Szx, nz)));
+    const float2 Sy = fma2(Sxy, nx, fma2(Syy, ny, mul2(Syz, nz)));
+    const float2 Sz = fma2(Szx, nx, fma2(Syz, ny, mul2(Szz, nz)));
+    const float2 u = fma2(nx, Sx, fma2(ny, Sy, mul2(nz, Sz)));
+    q = bl[2];
+    const float2 Dx = make_float2(q.x, q.y), Dy = make_float2(q.z, q.w);
+    q = bl[3];
+    const float2 Dz = make_float2(q.x, q.y), Qi = make_float2(q.z, q.w);
+    const float2 s15 = mul2(f2(1.5f), s), s2x = add2(s, s);
+    Wx = fma2(s2x, fma2(s15, Wx, Sx), Dx);
+    Wy = fma2(s2x, fma2(s15, Wy, Sy), Dy);
+    Wz = fma2(s2x, fma2(s15, Wz, Sz), Dz);
+    const float2 Dn = fma2(Dx, nx, fma2(Dy, ny, mul2(Dz, nz)));
+    ph = fma2(s, fma2(s, fma2(s, ph, u), Dn), Q);
+    w = fma2(s2x, fma2(s15, w, u), Dn);
+    const float2 s2 = mul2(s, s);
+    const float2 g = mul2(s2, fma2(s2x, w, ph));
+    const float2 ms3 = mul2(s2, mul2(f2(-1.f), s));
+    fx = fma2(g, nx, fma2(ms3, Wx, fx));
+    fy = fma2(g, ny, fma2(ms3, Wy, fy));
+    fz = fma2(g, nz, fma2(ms3, Wz, fz));
+    pa = fma2(s, ph, pa);
     pi = fma2(Qi, s, pi);
   }
   __syncwarp();
@@ -1143,7 +1114,7 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
         p2h += 32;
       }
       while (m2t - m2h >= 32) {
-        if (RDF) eval_m2p_x2<ORDER>(sm, m2h, 32, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
+        if (RDF || LEARNED) eval_m2p_x2<ORDER>(sm, m2h, 32, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
         else eval_m2p<ORDER>(sm, m2h, 32, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
         m2h += 32;
       }
@@ -1161,7 +1132,7 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
                           tly, tlz, close2, pt, tsp, act, lane, hist, acc);
     }
     if (m2t > m2h) {
-      if (RDF) eval_m2p_x2<ORDER>(sm, m2h, m2t - m2h, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
+      if (RDF || LEARNED) eval_m2p_x2<ORDER>(sm, m2h, m2t - m2h, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
       else eval_m2p<ORDER>(sm, m2h, m2t - m2h, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
     }
     if (lct > lch) {
