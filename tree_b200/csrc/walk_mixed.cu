@@ -583,62 +583,67 @@ __device__ __forceinline__ void rdf_count2(const MixedArgs& a, uint32_t* hist, f
   if (ok1 && t1 < (float)kRdfBins) atomicAdd(&hist[(same1 ? kRdfBins : 0) + (int)t1], 1u);
 }
 
+// hist[...] += 1 at a shared-memory address.
+__device__ __forceinline__ void rdf_inc(uint32_t at) {
+  asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory");
+}
+
 // One source against this lane's target with every case of the pair laws:
 // "special" pairs leave the plain Coulomb law -- the target itself (r = 0),
 // pairs inside the Kelbg core (exp(-x^2) still visible in FP32), and for the
 // reference laws same-species pairs inside the r^2 <= 0.01 cutoff and e-i
 // pairs where exp(-r/rs) is visible.
 template <int PHYS>
+__device__ __noinline__ float2 p2p_special(float r2, float ssign, float il, float rs_inv) {
+  // (force over separation, potential) of a special pair that interacts
+  float fs = 0.f, ve;
+  if (PHYS == 1) {
+    const float sqrtpi = 1.77245385f;
+    if (r2 > 0.f) {
+      const float r = sqrtf(r2);
+      const float ri = 1.f / r;
+      const float x2 = r2 * il * il;
+      const float g = -expm1f(-x2);
+      fs = ssign * g * ri * ri * ri;
+      ve = g * ri + sqrtpi * erfcf(r * il) * il;
+    } else {
+      ve = sqrtpi * il;  // distinct particles on one point: V(0)
+    }
+  } else if (r2 > 0.f) {
+    const float r = sqrtf(r2);
+    const float ri = 1.f / r;
+    const float e = expf(-r * rs_inv);
+    const float g = ri - e * (ri + rs_inv);
+    fs = ssign * g * ri * ri;
+    ve = (1.f - e) * ri;
+  } else {
+    ve = rs_inv;  // r -> 0 limit of (1 - exp(-r/rs))/r
+  }
+  return make_float2(fs, ssign * ve);
+}
+
+template <int PHYS>
 __device__ __forceinline__ void p2p_one(const WarpSmem& sm, float r2, float dx, float dy,
                                         float dz, float ssign, int s, int p_self, int tsp,
                                         float& fx, float& fy, float& fz, float& pa,
                                         float& pq) {
   const bool same = ssign == (tsp ? 1.f : -1.f);
-  const float il2_same = PHYS == 1 ? (tsp ? sm.pk[2] : sm.pk[0]) : 0.f;
-  const float il_same = PHYS == 1 ? (tsp ? sm.pk[6] : sm.pk[4]) : 0.f;
-  const float il2_ei = sm.pk[1], il_ei = sm.pk[5], rs_inv = sm.pk[3];
+  const float il2 = PHYS == 1 ? (same ? (tsp ? sm.pk[2] : sm.pk[0]) : sm.pk[1]) : 0.f;
+  const float rs_inv = sm.pk[3];
   bool special;
-  if (PHYS == 1) special = r2 * (same ? il2_same : il2_ei) < 40.f;
+  if (PHYS == 1) special = r2 * il2 < 40.f;
   else special = same ? !(r2 > 0.01f) : r2 * (rs_inv * rs_inv) < 400.f;
-  float fs, ph;
+  float fs = 0.f, ph = 0.f;
   if (!special) {
     const float rinv = rsqrtf(r2);
     fs = ssign * rinv * rinv * rinv;
     ph = ssign * rinv;
-  } else {
-    fs = 0.f;
-    ph = 0.f;
-    if (PHYS == 1) {
-      if (s != p_self) {
-        const float il = same ? il_same : il_ei;
-        const float sqrtpi = 1.77245385f;
-        float ve;
-        if (r2 > 0.f) {
-          const float r = sqrtf(r2);
-          const float ri = 1.f / r;
-          const float x2 = r2 * il * il;
-          const float g = -expm1f(-x2);
-          fs = ssign * g * ri * ri * ri;
-          ve = g * ri + sqrtpi * erfcf(r * il) * il;
-        } else {
-          ve = sqrtpi * il;  // distinct particles on one point: V(0)
-        }
-        ph = ssign * ve;
-      }
-    } else if (!same) {
-      float ve;
-      if (r2 > 0.f) {
-        const float r = sqrtf(r2);
-        const float ri = 1.f / r;
-        const float e = expf(-r * rs_inv);
-        const float g = ri - e * (ri + rs_inv);
-        fs = ssign * g * ri * ri;
-        ve = (1.f - e) * ri;
-      } else {
-        ve = rs_inv;  // r -> 0 limit of (1 - exp(-r/rs))/r
-      }
-      ph = ssign * ve;
-    }  // same species inside the cutoff (and the target itself): nothing
+  } else if (PHYS == 1 ? s != p_self : !same) {
+    // the target itself, and same species inside the cutoff: nothing
+    const float il = PHYS == 1 ? (same ? (tsp ? sm.pk[6] : sm.pk[4]) : sm.pk[5]) : 0.f;
+    const float2 v = p2p_special<PHYS>(r2, ssign, il, rs_inv);
+    fs = v.x;
+    ph = v.y;
   }
   fx = fmaf(fs, dx, fx);
   fy = fmaf(fs, dy, fy);
@@ -660,7 +665,7 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, int head, int cnt,
                                          int p_self, int tsp, bool act, int lane,
                                          uint32_t* hist, Acc& acc) {
   {
-    // this lane's source (or, past cnt, a chargeless dummy 10^6 um away)
+    // this lane's source (or, past cnt, a chargeless dummy beyond any RDF bin)
     float v[8];
     if (lane < cnt) {
       const int s = sm.p2p[(head + lane) & (kP2pRing - 1)];
@@ -671,7 +676,7 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, int head, int cnt,
       v[4] = (float)(rx - (double)hx); v[5] = (float)(ry - (double)hy);
       v[6] = (float)(rz - (double)hz); v[7] = __int_as_float(s);
     } else {
-      v[0] = v[1] = v[2] = 1.0e6f;
+      v[0] = v[1] = v[2] = 1.0e18f;
       v[3] = 0.f;
       v[4] = v[5] = v[6] = 0.f;
       v[7] = __int_as_float(-1);
@@ -688,14 +693,33 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, int head, int cnt,
   }
   __syncwarp();
   // the source charge that makes a pair "same species" for this target, and
-  // the FP32 screening constants of the common-path test
+  // the FP32 screening constants of the special-pair test
   const float tq = tsp ? 1.f : -1.f;
   const float il2_to_e = PHYS == 1 ? (tsp ? sm.pk[1] : sm.pk[0]) : 0.f;  // electron source
   const float il2_to_i = PHYS == 1 ? (tsp ? sm.pk[2] : sm.pk[1]) : 0.f;  // ion source
   const float rs2 = sm.pk[3] * sm.pk[3];
+  // one test sends a pair to the exact offsets or a special law: the largest
+  // squared distance at which any of them could apply (1.01: its rounding)
+  const float near2 =
+      fmaxf(close2, 1.01f * (PHYS == 1 ? 40.f / fminf(il2_to_e, il2_to_i)
+                                       : fmaxf(0.01f, 400.f / rs2)));
+  // RDF counts of the other pairs: bin = trunc(r * rdf_inv), read off the low
+  // bits of r * rdf_inv + 2^23 (rounded towards zero; + the ii histogram's
+  // offset); a scale of 1e30 puts pairs that are not counted (electrons for an
+  // electron target, every pair of an idle lane) beyond the last bin
+  float inv_i = 1e30f, inv_e = 1e30f, bin_i = 8388608.f;
+  uint32_t hist_at = 0;
+  if (RDF) {
+    if (act) inv_i = tsp ? a.dx_ii_inv_f : a.dx_ei_inv_f;
+    if (act && tsp) inv_e = a.dx_ei_inv_f;
+    if (tsp) bin_i += (float)kRdfBins;
+    // (0x4B000000 + bin) * 4 + hist_at = address of the bin, modulo 2^32
+    hist_at = (uint32_t)__cvta_generic_to_shared(hist) - (0x4B000000u << 2);
+  }
   const float2 thx2 = make_float2(thx, thx), thy2 = make_float2(thy, thy), thz2 = make_float2(thz, thz);
   float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx, pa = fx, pq = fx;
   const int npair = (cnt + 1) >> 1;
+#pragma unroll 1
   for (int b = 0; b < npair; ++b) {
     const float4* blk = sm.part + kPartF4 * b;
     const float4 q0 = blk[0], q1 = blk[1];
@@ -704,6 +728,26 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, int head, int cnt,
     float2 dy = __fadd2_rn(thy2, make_float2(q0.z, q0.w));
     float2 dz = __fadd2_rn(thz2, make_float2(q1.x, q1.y));
     float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    if (fminf(r2.x, r2.y) > near2) {
+      const float2 rinv = make_float2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
+      const float2 ph = __fmul2_rn(q, rinv);
+      const float2 fs = __fmul2_rn(ph, __fmul2_rn(rinv, rinv));
+      fx = __ffma2_rn(fs, dx, fx);
+      fy = __ffma2_rn(fs, dy, fy);
+      fz = __ffma2_rn(fs, dz, fz);
+      pa = __fadd2_rn(pa, ph);
+      pq = __ffma2_rn(q, ph, pq);
+      if (RDF) {
+        const bool i0 = q.x > 0.f, i1 = q.y > 0.f;
+        const float2 t = __fmul2_rn(__fmul2_rn(r2, rinv),
+                                    make_float2(i0 ? inv_i : inv_e, i1 ? inv_i : inv_e));
+        const float b0 = __fadd_rz(t.x, i0 ? bin_i : 8388608.f);
+        const float b1 = __fadd_rz(t.y, i1 ? bin_i : 8388608.f);
+        if (t.x < (float)kRdfBins) rdf_inc(hist_at + 4u * __float_as_uint(b0));
+        if (t.y < (float)kRdfBins) rdf_inc(hist_at + 4u * __float_as_uint(b1));
+      }
+      continue;
+    }
     int s0 = -1, s1 = -1;
     if (r2.x <= close2 || r2.y <= close2) {
       // close pair: the exact offsets (hi + lo) and the source indices
@@ -966,7 +1010,8 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
     float lsum = 0.f;  // lanes 0..19: one summed coefficient of the local expansion
     bool overflow = false;
     int cqh = 0, cqt = 0;  // learned-MAC candidate ring (warp-uniform)
-    while (ssize > 0 || cqt > cqh) {
+    bool fin = false;
+    while (!fin) {
       int node = -1;
       int action = 0, pfirst = 0, pcnt = 0;  // 1 far field, 2 particles, 3 open
       if (LEARNED && (cqt - cqh >= 32 || (ssize == 0 && cqt > cqh))) {
@@ -1108,35 +1153,31 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
       ssize += ktot;
       max_stack = max(max_stack, ssize);
       __syncwarp();
-      while (p2t - p2h >= 32) {
-        eval_p2p<PHYS, RDF>(sm, p2h, 32, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, tlx, tly,
-                            tlz, close2, pt, tsp, act, lane, hist, acc);
-        p2h += 32;
+      // Full batches of 32, and what is left once the walk has ended.  One
+      // call site each: the evaluations are long straight-line code, and the
+      // warps of an SM are in different ones.
+      fin = ssize == 0 && cqt == cqh;
+      while (p2t - p2h >= 32 || (fin && p2t > p2h)) {
+        const int cnt = min(32, p2t - p2h);
+        eval_p2p<PHYS, RDF>(sm, p2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, tlx, tly, tlz,
+                            close2, pt, tsp, act, lane, hist, acc);
+        p2h += cnt;
       }
-      while (m2t - m2h >= 32) {
-        if (RDF || LEARNED) eval_m2p_x2<ORDER>(sm, m2h, 32, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
-        else eval_m2p<ORDER>(sm, m2h, 32, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
-        m2h += 32;
+      while (m2t - m2h >= 32 || (fin && m2t > m2h)) {
+        const int cnt = min(32, m2t - m2h);
+        if (RDF || LEARNED) eval_m2p_x2<ORDER>(sm, m2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
+        else eval_m2p<ORDER>(sm, m2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
+        m2h += cnt;
       }
-      while (lct - lch >= 32) {
-        eval_local<ORDER>(sm, lch, 32, a, sm.gx, sm.gy, sm.gz, lane, lsum);
-        lch += 32;
+      while (lct - lch >= 32 || (fin && lct > lch)) {
+        const int cnt = min(32, lct - lch);
+        eval_local<ORDER>(sm, lch, cnt, a, sm.gx, sm.gy, sm.gz, lane, lsum);
+        lch += cnt;
       }
     }
     if (overflow) {
       if (lane == 0) set_error(a.err, kErrWalk);
       continue;
-    }
-    if (p2t > p2h) {
-      eval_p2p<PHYS, RDF>(sm, p2h, p2t - p2h, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, tlx,
-                          tly, tlz, close2, pt, tsp, act, lane, hist, acc);
-    }
-    if (m2t > m2h) {
-      if (RDF || LEARNED) eval_m2p_x2<ORDER>(sm, m2h, m2t - m2h, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
-      else eval_m2p<ORDER>(sm, m2h, m2t - m2h, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
-    }
-    if (lct > lch) {
-      eval_local<ORDER>(sm, lch, lct - lch, a, sm.gx, sm.gy, sm.gz, lane, lsum);
     }
     if (lct > 0) {
       // every target evaluates the group's summed local expansion
