@@ -36,26 +36,24 @@
 
 namespace tg {
 
-constexpr int kMxWarps = 8;
-constexpr int kMxThreads = 32 * kMxWarps;
 constexpr int kStackCap = 8192;   // node indices per warp
 constexpr int kM2pRing = 64;      // power of two, > 31 + 32
 constexpr int kLocRing = 64;      // power of two, > 31 + 32
 constexpr int kLocStride = kLocCoef | 1;  // odd row stride of the coefficient rows
-constexpr int kP2pRing = 512;     // power of two, > 31 + 32 * kMaxBucket
 constexpr int kMaxBucket = 8;
+constexpr int kP2pBuf = 31 + 32 * kMaxBucket + 1;  // what a batch of nodes can leave
 constexpr int kMaxBlocksPerSm = 4;
-// Blocks per SM the walk without RDF counts is compiled for: the fixed test
-// at 3 (80 registers, 24 resident warps), the learned criterion at 2 (128
-// registers, 16 warps): its candidate ring and budget make the 80-register
-// build spill, which cost 13 % of its walk at N = 1M (23.1 against 20.4 ms),
-// while the fixed test runs 5 % faster at 80 registers than at 128.
-constexpr int kMinBlocksPerSm = 3;
-constexpr int kMinBlocksPerSmLearned = 2;
-// With RDF counts the walk runs one block of kRdfWarps per SM that keeps both
-// histograms (2 x 10001 u32) in shared memory and adds them to the global
-// bins once, when the block ends.
-constexpr int kRdfWarps = 16;
+// One block per SM.  The fixed test without RDF counts runs 20 warps of 96
+// registers: N = 1M takes 10.75 ms, against 11.1 ms for 16 warps of 128 and
+// 11.9 ms for 24 of 80, whose far field had to go one cell at a time and
+// spilled.  The learned criterion's build runs 16 warps of 128 (20 of 96: 1.4 %
+// slower at N = 4M, 0.6 % faster on the ensemble; 24 of 80: 7 to 24 % slower),
+// and so do the builds with RDF counts, whose histograms (2 x 10001 u32, added
+// to the global bins once, when the block ends) leave no room for more.
+constexpr int kWarpStep = 8;      // warps per unit of the blocks_per_sm tunable
+constexpr int kStackWarps = 32;   // per SM: stacks of the walk's and the sampler's warps
+template <bool RDF, bool LEARNED>
+constexpr int walk_warps() { return RDF || LEARNED ? 16 : 20; }
 
 constexpr int kCandRing = 64;     // power of two, > 31 + 32
 constexpr int kCellF4 = 9;        // float4 per staged far-field cell (order 4)
@@ -64,7 +62,7 @@ constexpr int kPartF4 = 5;        // float4 per staged source pair (4 used + pad
 struct WarpSmem {
   int m2p[kM2pRing];
   int loc[kLocRing];       // far cells summed into the group's local expansion
-  int p2p[kP2pRing];
+  int p2p[kP2pBuf];        // particle entries; at most 31 between batches
   int cq_node[kCandRing];  // learned-MAC candidates waiting for a full batch
   // The far-field and pair staging areas (and the learned MAC's feature
   // rows, in `cell`) are used one at a time by the warp: one buffer.
@@ -251,114 +249,22 @@ __device__ __forceinline__ void m2p_rows(const MixedArgs& a, int node, double Gx
   }
 }
 
-template <int ORDER>
-__device__ __forceinline__ void eval_m2p(WarpSmem& sm, int head, int cnt,
-                                         const MixedArgs& a, double Gx,
-                                         double Gy, double Gz, float tx,
-                                         float ty, float tz, int lane,
-                                         Acc& acc) {
-  constexpr int kRows = ORDER >= 4 ? 9 : (ORDER == 3 ? 6 : 4);
-  if (lane < cnt) {
-    float4 r[kRows];
-    m2p_rows<ORDER>(a, sm.m2p[(head + lane) & (kM2pRing - 1)], Gx, Gy, Gz, r);
-    float4* cl = sm.cell + kCellF4 * lane;
-#pragma unroll
-    for (int j = 0; j < kRows; ++j) cl[j] = r[j];
-  }
-  __syncwarp();
-  float fx = 0.f, fy = 0.f, fz = 0.f, pa = 0.f, pi = 0.f;
-#pragma unroll 1
-  for (int k = 0; k < cnt; ++k) {
-    const float4* cl = sm.cell + kCellF4 * k;
-    const float4 A = cl[0];
-    const float dx = tx + A.x, dy = ty + A.y, dz = tz + A.z;
-    // accepted cells are farther than rcrit >= 0; the 1e-30 only guards a
-    // zero-size cell against an FP32 distance of 0
-    const float s = rsqrt_normal(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 1e-30f))));
-    const float nx = dx * s, ny = dy * s, nz = dz * s;
-    const float xx = nx * nx, yy = ny * ny, zz = nz * nz;
-    const float a2 = xx - zz, b2 = yy - zz;
-    float Wx = 0.f, Wy = 0.f, Wz = 0.f, ph = 0.f, w = 0.f;
-    const float4 E = cl[3];
-    if (ORDER >= 4) {
-      const float4 H0 = cl[6], H1 = cl[7], H2 = cl[8];
-      const float x3 = 3.f * nx, y3 = 3.f * ny;
-      const float P1 = nx * fmaf(-3.f, zz, xx), P6 = ny * fmaf(-3.f, zz, yy);
-      const float P2 = y3 * a2, P4 = x3 * b2;
-      const float P3 = nz * fmaf(3.f, xx, -zz), P7 = nz * fmaf(3.f, yy, -zz);
-      const float P5 = x3 * (2.f * ny * nz);
-      // (xxxx xxxy xxxz xxyy) (xxyz xyyy xyyz yyyy) (yyyz xxzz xyzz yyzz)
-      Wx = fmaf(H0.x, P1, fmaf(H0.y, P2, fmaf(H0.z, P3, fmaf(H0.w, P4,
-           fmaf(H1.x, P5, fmaf(H1.y, P6, H1.z * P7))))));
-      Wy = fmaf(H0.y, P1, fmaf(H0.w, P2, fmaf(H1.x, P3, fmaf(H1.y, P4,
-           fmaf(H1.z, P5, fmaf(H1.w, P6, H2.x * P7))))));
-      Wz = fmaf(H0.z, P1, fmaf(H1.x, P2, fmaf(H2.y, P3, fmaf(H1.z, P4,
-           fmaf(H2.z, P5, fmaf(H2.x, P6, H2.w * P7))))));
-      ph = fmaf(nx, Wx, fmaf(ny, Wy, nz * Wz));
-      w = ph;
-    }
-    if (ORDER >= 3) {
-      // xxx = E.z, yyy = E.w, xxy = T1.y, xxz = T1.z, xyy = T1.w, yyz = T2.x,
-      // xzz = T2.y, yzz = T2.z, xyz = T2.w
-      const float4 T1 = cl[4], T2 = cl[5];
-      const float x2 = nx + nx, y2 = ny + ny;
-      const float xy2 = x2 * ny, xz2 = x2 * nz, yz2 = y2 * nz;
-      const float Tx = fmaf(E.z, a2, fmaf(T1.w, b2, fmaf(T1.y, xy2, fmaf(T1.z, xz2, T2.w * yz2))));
-      const float Ty = fmaf(T1.y, a2, fmaf(E.w, b2, fmaf(T1.w, xy2, fmaf(T2.w, xz2, T2.x * yz2))));
-      const float Tz = fmaf(T1.z, a2, fmaf(T2.x, b2, fmaf(T2.w, xy2, fmaf(T2.y, xz2, T2.z * yz2))));
-      const float t = fmaf(nx, Tx, fmaf(ny, Ty, nz * Tz));
-      const float s43 = (4.f / 3.f) * s;
-      Wx = fmaf(s43, Wx, Tx);
-      Wy = fmaf(s43, Wy, Ty);
-      Wz = fmaf(s43, Wz, Tz);
-      ph = fmaf(s, ph, t);
-      w = fmaf(s43, w, t);
-    }
-    const float4 B = cl[1], C = cl[2];
-    // S n with S = [[Sxx,Sxy,Szx],[Sxy,Syy,Syz],[Szx,Syz,Szz]]
-    const float Sx = fmaf(C.x, nx, fmaf(C.w, ny, E.y * nz));
-    const float Sy = fmaf(C.w, nx, fmaf(C.y, ny, E.x * nz));
-    const float Sz = fmaf(E.y, nx, fmaf(E.x, ny, C.z * nz));
-    const float u = fmaf(nx, Sx, fmaf(ny, Sy, nz * Sz));
-    const float s15 = 1.5f * s, s2x = s + s;
-    Wx = fmaf(s2x, fmaf(s15, Wx, Sx), B.x);
-    Wy = fmaf(s2x, fmaf(s15, Wy, Sy), B.y);
-    Wz = fmaf(s2x, fmaf(s15, Wz, Sz), B.z);
-    const float Dn = fmaf(B.x, nx, fmaf(B.y, ny, B.z * nz));
-    ph = fmaf(s, fmaf(s, fmaf(s, ph, u), Dn), A.w);
-    w = fmaf(s2x, fmaf(s15, w, u), Dn);
-    const float s2 = s * s, g = s2 * fmaf(s2x, w, ph), ms3 = -s * s2;
-    fx = fmaf(g, nx, fmaf(ms3, Wx, fx));
-    fy = fmaf(g, ny, fmaf(ms3, Wy, fy));
-    fz = fmaf(g, nz, fmaf(ms3, Wz, fz));
-    pa = fmaf(s, ph, pa);
-    pi = fmaf(B.w, s, pi);
-  }
-  __syncwarp();
-  kahan_add(acc.sx, acc.cx, fx);
-  kahan_add(acc.sy, acc.cy, fy);
-  kahan_add(acc.sz, acc.cz, fz);
-  phi_add(sm, lane, (double)pa, (double)pi);
-}
-
-// The same far field two cells at a time on the packed FP32 (f32x2) pipeline:
+// The far field runs two cells at a time on the packed FP32 (f32x2) pipeline:
 // cells 2b and 2b+1 are staged side by side, so one 16-byte shared load gives
-// two float2 operands and every multiply-add serves both cells.  Used where
-// the walk runs with 128 registers per thread (the RDF layout: one 16-warp
-// block per SM), which holds the doubled live state without spills.
+// two float2 operands and every multiply-add serves both cells.
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
 template <int ORDER>
-__device__ __forceinline__ void eval_m2p_x2(WarpSmem& sm, int head, int cnt,
+__device__ __forceinline__ void eval_m2p(WarpSmem& sm, int head, int cnt,
                                             const MixedArgs& a, double Gx, double Gy,
                                             double Gz, float tx, float ty, float tz,
                                             int lane, Acc& acc) {
   constexpr int kRows = ORDER >= 4 ? 9 : (ORDER == 3 ? 6 : 4);
   {
-    // this lane's cell as kRows float4 rows (the layout of eval_m2p), or a
+    // this lane's cell as kRows float4 rows (see WarpSmem::cell), or a
     // chargeless dummy far away past cnt
     float4 r[kRows];
     if (lane < cnt) {
@@ -668,7 +574,7 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, int head, int cnt,
     // this lane's source (or, past cnt, a chargeless dummy beyond any RDF bin)
     float v[8];
     if (lane < cnt) {
-      const int s = sm.p2p[(head + lane) & (kP2pRing - 1)];
+      const int s = sm.p2p[head + lane];
       const double4 xs = a.xs[s];
       const double rx = Gx - xs.x, ry = Gy - xs.y, rz = Gz - xs.z;
       const float hx = (float)rx, hy = (float)ry, hz = (float)rz;
@@ -870,32 +776,36 @@ __global__ void k_mac_node_terms(const float4* __restrict__ geom,
 
 // --------------------------------------------------------------- walk ----
 // Dynamic shared memory: WarpSmem per warp, then (learned MAC only) the
-// packed network and the features' training range, then (RDF only) the two
-// block histograms.
+// features' training range and, without RDF counts, the packed network, then
+// (RDF only) the two block histograms.  With RDF counts the network stays in
+// global memory: it is read once per 32 candidates, and its 11 KB bring the
+// block under the step at which the SM keeps 60 KB of L1 instead of 28 KB.
+constexpr size_t kFrangeBytes = sizeof(float) * (2 * kMacFeatures + 8);
+template <bool LEARNED, bool RDF>
 constexpr size_t walk_learned_bytes() {
-  return (sizeof(MlpPacked) + sizeof(float) * (2 * kMacFeatures + 8) + 15) / 16 * 16;
+  return LEARNED ? (kFrangeBytes + (RDF ? 0 : sizeof(MlpPacked)) + 15) / 16 * 16 : 0;
 }
 template <bool LEARNED, bool RDF>
-constexpr size_t walk_smem_bytes() {
-  return sizeof(WarpSmem) * (RDF ? kRdfWarps : kMxWarps) + (LEARNED ? walk_learned_bytes() : 0) +
+constexpr size_t walk_smem_bytes(int warps) {
+  return sizeof(WarpSmem) * warps + walk_learned_bytes<LEARNED, RDF>() +
          (RDF ? sizeof(uint32_t) * 2 * kRdfBins : 0);
 }
-
-// the largest variant must fit one block's opt-in shared memory (227 KB)
-static_assert(walk_smem_bytes<true, true>() <= 232448, "walk shared memory over 227 KB");
-static_assert(walk_smem_bytes<true, false>() * kMinBlocksPerSm <= 233472 - 3 * 1024,
-              "three walk blocks no longer fit one SM");
+static_assert(walk_smem_bytes<true, true>(16) <= 195 * 1024, "RDF walk over the 196 KB step");
+static_assert(walk_smem_bytes<false, false>(20) <= 163 * 1024, "walk over the 164 KB step");
 
 template <int PHYS, bool RDF, bool LEARNED, int ORDER>
-__global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
-                                  RDF ? 1 : (LEARNED ? kMinBlocksPerSmLearned : kMinBlocksPerSm))
-    k_walk_mixed(MixedArgs a) {
-  constexpr int kW = RDF ? kRdfWarps : kMxWarps;
+__global__ void __launch_bounds__(32 * walk_warps<RDF, LEARNED>(), 1) k_walk_mixed(MixedArgs a) {
   extern __shared__ float4 dyn_smem[];
   WarpSmem* smem = reinterpret_cast<WarpSmem*>(dyn_smem);
-  unsigned char* tail = reinterpret_cast<unsigned char*>(smem + kW);
-  MlpPacked* mlp = reinterpret_cast<MlpPacked*>(tail);
-  uint32_t* hist = reinterpret_cast<uint32_t*>(tail + (LEARNED ? walk_learned_bytes() : 0));
+  const int nwarps = blockDim.x >> 5;
+  unsigned char* tail = reinterpret_cast<unsigned char*>(smem + nwarps);
+  // training range of the features (fmin | fmax), then m_lo, m_hi and the
+  // pre-filter coefficients, shared by the block
+  float* frange = reinterpret_cast<float*>(tail);
+  const float* fmodel = frange + 2 * kMacFeatures;
+  MlpPacked* mlp_s = reinterpret_cast<MlpPacked*>(tail + kFrangeBytes);
+  const MlpPacked* mlp = RDF ? a.packed : mlp_s;
+  uint32_t* hist = reinterpret_cast<uint32_t*>(tail + walk_learned_bytes<LEARNED, RDF>());
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   WarpSmem& sm = smem[wib];
@@ -904,16 +814,11 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
     __syncthreads();
   }
   if (LEARNED) {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(a.packed);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(mlp);
-    for (int i = threadIdx.x; i < (int)(sizeof(MlpPacked) / 4); i += blockDim.x) dst[i] = src[i];
-    __syncthreads();
-  }
-  // training range of the features (fmin | fmax), then m_lo, m_hi and the
-  // pre-filter coefficients, shared by the block
-  float* frange = reinterpret_cast<float*>(mlp + 1);
-  const float* fmodel = frange + 2 * kMacFeatures;
-  if (LEARNED) {
+    if (!RDF) {
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(a.packed);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(mlp_s);
+      for (int i = threadIdx.x; i < (int)(sizeof(MlpPacked) / 4); i += blockDim.x) dst[i] = src[i];
+    }
     if (threadIdx.x < kMacFeatures) {
       frange[threadIdx.x] = __ldg(&a.fmin[threadIdx.x]);
       frange[kMacFeatures + threadIdx.x] = __ldg(&a.fmax[threadIdx.x]);
@@ -922,17 +827,22 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
       frange[2 * kMacFeatures + threadIdx.x] = __ldg(&a.margins[threadIdx.x]);
     __syncthreads();
   }
-  const int gwarp = blockIdx.x * kW + wib;
+  const int gwarp = blockIdx.x * nwarps + wib;
   int32_t* stack = a.stack + (int64_t)gwarp * kStackCap;
   const unsigned lt = (1u << lane) - 1u;
   if (*((volatile int32_t*)a.err) & (kErrCapacity | kErrDepth | kErrNonFinite)) return;
   const int root_end = a.bounds[2];  // combined tree: nodes [0, root_end)
   const int ngroups = *a.n_groups;
   int max_stack = 0;
-  while (root_end > 0) {
-    int g = 0;
-    if (lane == 0) g = atomicAdd(&a.control[0], 1);
-    g = __shfl_sync(0xffffffffu, g, 0);
+  // The first group of each warp is fixed, spread over the SMs before the warps
+  // of an SM: with fewer groups than warps, a cursor alone gives them all to
+  // the blocks that start first (N = 32,768 kept 55 of the 148 SMs busy).
+  int g = wib * gridDim.x + blockIdx.x;
+  for (bool own = true; root_end > 0; own = false) {
+    if (!own) {
+      if (lane == 0) g = gridDim.x * nwarps + atomicAdd(&a.control[0], 1);
+      g = __shfl_sync(0xffffffffu, g, 0);
+    }
     if (g >= ngroups) break;
     const int2 grp = a.groups[g];
     const int p0 = grp.x, n_act = grp.y;
@@ -1005,7 +915,8 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
     }
     if (lane == 0) stack[0] = root;
     __syncwarp();
-    int m2h = 0, m2t = 0, p2h = 0, p2t = 0;  // ring heads/tails (warp-uniform)
+    int m2h = 0, m2t = 0;  // ring head/tail (warp-uniform)
+    int p2n = 0, p2tot = 0;  // particle entries waiting, evaluated
     int lch = 0, lct = 0;                    // local-expansion ring
     float lsum = 0.f;  // lanes 0..19: one summed coefficient of the local expansion
     bool overflow = false;
@@ -1125,8 +1036,8 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
       const int pex = warp_excl_scan(action == 2 ? pcnt : 0, lane, &ptot);
       if (action == 2)
         for (int k = 0; k < pcnt; ++k)
-          sm.p2p[(p2t + pex + k) & (kP2pRing - 1)] = pfirst + k;
-      p2t += ptot;
+          sm.p2p[p2n + pex + k] = pfirst + k;
+      p2n += ptot;
       // opened twigs push their children (octant order)
       int4 k0 = make_int4(-1, -1, -1, -1), k1 = k0;
       if (action == 3) {
@@ -1157,16 +1068,24 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
       // call site each: the evaluations are long straight-line code, and the
       // warps of an SM are in different ones.
       fin = ssize == 0 && cqt == cqh;
-      while (p2t - p2h >= 32 || (fin && p2t > p2h)) {
-        const int cnt = min(32, p2t - p2h);
+      int p2h = 0;
+      while (p2n - p2h >= 32 || (fin && p2n > p2h)) {
+        const int cnt = min(32, p2n - p2h);
         eval_p2p<PHYS, RDF>(sm, p2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, tlx, tly, tlz,
                             close2, pt, tsp, act, lane, hist, acc);
         p2h += cnt;
       }
+      if (p2h > 0) {  // the remainder moves to the front
+        p2tot += p2h;
+        p2n -= p2h;
+        const int e = lane < p2n ? sm.p2p[p2h + lane] : 0;
+        __syncwarp();
+        if (lane < p2n) sm.p2p[lane] = e;
+        __syncwarp();
+      }
       while (m2t - m2h >= 32 || (fin && m2t > m2h)) {
         const int cnt = min(32, m2t - m2h);
-        if (RDF || LEARNED) eval_m2p_x2<ORDER>(sm, m2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
-        else eval_m2p<ORDER>(sm, m2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
+        eval_m2p<ORDER>(sm, m2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
         m2h += cnt;
       }
       while (lct - lch >= 32 || (fin && lct > lch)) {
@@ -1207,7 +1126,7 @@ __global__ void __launch_bounds__(RDF ? 32 * kRdfWarps : kMxThreads,
     if (lane == 0) {
       // every queued entry was evaluated: the ring tails are the counts
       atomicAdd(&a.counters[0], (unsigned long long)m2t * n_act);
-      atomicAdd(&a.counters[1], (unsigned long long)p2t * n_act);
+      atomicAdd(&a.counters[1], (unsigned long long)p2tot * n_act);
       if (lct > 0) atomicAdd(&a.counters[8], (unsigned long long)lct);
     }
     if (LEARNED) {
@@ -1260,7 +1179,8 @@ int mixed_alloc_particles(MixedBuffers& mb, int n) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  mb.grid_warps = sms * kMaxBlocksPerSm * kMxWarps;
+  mb.sms = sms;
+  mb.grid_warps = sms * kStackWarps;
   int rc = 0;
   rc |= realloc_dev(&mb.xs, (size_t)n);
   rc |= realloc_dev(&mb.groups, (size_t)n);
@@ -1368,14 +1288,11 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
   a.ens_start = ens.start;
   a.roots = ens.roots;
   a.cloud_pk = cloud_pk;
-  int bps = tune.blocks_per_sm < 1 ? 1 : (tune.blocks_per_sm > kMaxBlocksPerSm ? kMaxBlocksPerSm : tune.blocks_per_sm);
-  // the learned build holds at most kMinBlocksPerSmLearned blocks per SM:
-  // more would only queue behind them
-  if (L && bps > kMinBlocksPerSmLearned) bps = kMinBlocksPerSmLearned;
-  const int sms_grid = mb.grid_warps / (kMaxBlocksPerSm * kMxWarps);
-  int grid = sms_grid * bps;
+  // warps per SM: kWarpStep per unit of blocks_per_sm, up to what the build
+  // holds (a fixed 16 with RDF counts)
+  const int bps = tune.blocks_per_sm < 1 ? 1 : (tune.blocks_per_sm > kMaxBlocksPerSm ? kMaxBlocksPerSm : tune.blocks_per_sm);
   const bool r = rdf != nullptr;
-  if (L) k_mac_node_terms<<<sms_grid * 4, 256, 0, st>>>(mb.geom, mb.mom3, tv.tree_bounds,
+  if (L) k_mac_node_terms<<<mb.sms * 4, 256, 0, st>>>(mb.geom, mb.mom3, tv.tree_bounds,
                                                        learned->margins, 1.f / learned->rho_hi,
                                                        mb.mac_k);
   int dev = 0;
@@ -1383,14 +1300,16 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
 #define TG_LAUNCH(P, R, LL, O)                                                \
   do {                                                                        \
     auto kfn = k_walk_mixed<P, R, LL, O>;                                     \
-    const size_t sb = walk_smem_bytes<LL, R>();                               \
+    const int most = walk_warps<R, LL>();                                     \
+    const int nw = R || kWarpStep * bps > most ? most : kWarpStep * bps;      \
+    const size_t sb = walk_smem_bytes<LL, R>(nw);                             \
     static unsigned attr_set = 0; /* devices with the smem limit raised */    \
     if (dev < 32 && !(attr_set & (1u << dev))) {                              \
       cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                           (int)sb);                                          \
+                           (int)walk_smem_bytes<LL, R>(most));                \
       attr_set |= 1u << dev;                                                  \
     }                                                                         \
-    kfn<<<R ? sms_grid : grid, R ? 32 * kRdfWarps : kMxThreads, sb, st>>>(a); \
+    kfn<<<mb.sms, 32 * nw, sb, st>>>(a);                                      \
   } while (0)
 #define TG_LAUNCH_O(P, R, LL)                                                 \
   do {                                                                        \

@@ -29,13 +29,14 @@ struct MixedBuffers {
   int32_t* cls = nullptr;      // net pass: class counts per node block, then their scan
   int32_t* stack = nullptr;    // per resident warp: kStackCap node indices
   int32_t* control = nullptr;  // [0] group cursor, [1] max stack depth, [2] groups
-  int grid_warps = 0;
+  int sms = 0;                 // SMs of the device: one walk block each
+  int grid_warps = 0;          // warps with a stack
 };
 
 // Tunables of the walk (picked by tree_b200/tune.py; defaults below).
 struct MixedTuning {
   int bucket = 8;          // twigs with <= bucket particles are summed directly
-  int blocks_per_sm = 4;   // persistent grid: SMs x blocks_per_sm blocks
+  int blocks_per_sm = 4;   // warps per SM in units of 8, up to what the build holds
   int order = 3;           // far-field order: 2 quadrupole, 3 octupole, 4 hexadecapole
   // accepted cells far from a target group are summed into the group's local
   // expansion (local.cuh) when (group half-diagonal) / (distance from the
