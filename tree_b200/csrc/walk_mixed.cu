@@ -55,6 +55,18 @@ constexpr int kStackWarps = 32;   // per SM: stacks of the walk's and the sample
 template <bool RDF, bool LEARNED>
 constexpr int walk_warps() { return RDF || LEARNED ? 16 : 20; }
 
+// Warps that share a group.  Below about 20,000 particles there are fewer
+// groups (of about 25 targets) than half the warps of the GPU, and a group is a
+// serial walk; a team's leader walks, and its warps evaluate the same batches
+// that one warp would, in rounds, so the forces are the same to the last bit.
+// Walk ms for 1, 4, 8, 16 warps (hexadecapole, theta 0.42, fixed | with RDF):
+//   N = 1,000   0.098 0.063 0.057 0.053 | 0.131 0.080 0.069 0.064
+//   N = 4,096   0.280 0.171 0.151 0.184 | 0.349 0.192 0.164 0.200
+//   N = 8,192   0.422 0.261 0.290 0.377 | 0.517 0.291 0.315 0.402
+//   N = 16,384  0.553 0.468 0.551 0.793 | 0.609 0.501 0.599 0.836
+//   N = 32,768  0.895 0.908 1.196 1.843 | 0.947 0.990 1.297 1.959
+int walk_team(int n) { return n < 3000 ? 16 : (n < 6000 ? 8 : (n < 20000 ? 4 : 1)); }
+
 constexpr int kCandRing = 64;     // power of two, > 31 + 32
 constexpr int kCellF4 = 9;        // float4 per staged far-field cell (order 4)
 constexpr int kPartF4 = 5;        // float4 per staged source pair (4 used + pad)
@@ -105,6 +117,16 @@ __device__ __forceinline__ void phi_add(WarpSmem& sm, int lane, double all, doub
   sm.phi[lane] = p;
 }
 
+// A team of warps and its queue of batches: the leader walks and fills it, every
+// warp evaluates one batch a round, the leader adds the results in order.
+constexpr int kTeamMin = 4;
+constexpr int kTeamQueue = 15 + 13;  // one short of the largest team, and what a walk's end adds
+struct TeamSmem {
+  int item, take;            // the team's group; batches of this round (0: group done)
+  int info[kTeamQueue];      // 4 * entries + kind: 1 far field, 2 particles, 3 local
+  int idx[kTeamQueue][32];
+};
+
 struct MixedArgs {
   const double4* __restrict__ node_c;
   const float4* __restrict__ mom;
@@ -119,6 +141,7 @@ struct MixedArgs {
   int n, n_el;
   int32_t* control;
   int32_t* stack;
+  int team;  // warps that share a group (TEAM builds; a power of two)
   int bucket;
   int p2p_max;  // accepted cells with at most this many particles go to P2P
   // accepted cells far from the group go to its local expansion: h / d <=
@@ -165,11 +188,25 @@ struct Acc {
   // once per batch of 32 entries and need not hold registers in between.
 };
 
+// What one batch of 32 entries gives this lane: unscaled force and potential
+// (all sources, ion part) of its target, or one local-expansion coefficient.
+struct alignas(16) Batch {
+  float fx, fy, fz, loc;
+  double pa, pi;
+};
+
 __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
   float y = v - c;
   float t = s + y;
   c = (t - s) - y;
   s = t;
+}
+
+__device__ __forceinline__ void batch_add(WarpSmem& sm, int lane, Acc& acc, const Batch& b) {
+  kahan_add(acc.sx, acc.cx, b.fx);
+  kahan_add(acc.sy, acc.cy, b.fy);
+  kahan_add(acc.sz, acc.cz, b.fz);
+  phi_add(sm, lane, b.pa, b.pi);
 }
 
 __device__ __forceinline__ int warp_excl_scan(int v, int lane, int* total) {
@@ -258,17 +295,17 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
 template <int ORDER>
-__device__ __forceinline__ void eval_m2p(WarpSmem& sm, int head, int cnt,
+__device__ __forceinline__ void eval_m2p(WarpSmem& sm, const int* list, int mask, int head, int cnt,
                                             const MixedArgs& a, double Gx, double Gy,
                                             double Gz, float tx, float ty, float tz,
-                                            int lane, Acc& acc) {
+                                            int lane, Batch& out) {
   constexpr int kRows = ORDER >= 4 ? 9 : (ORDER == 3 ? 6 : 4);
   {
     // this lane's cell as kRows float4 rows (see WarpSmem::cell), or a
     // chargeless dummy far away past cnt
     float4 r[kRows];
     if (lane < cnt) {
-      m2p_rows<ORDER>(a, sm.m2p[(head + lane) & (kM2pRing - 1)], Gx, Gy, Gz, r);
+      m2p_rows<ORDER>(a, list[(head + lane) & mask], Gx, Gy, Gz, r);
     } else {
       r[0] = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f);
 #pragma unroll
@@ -392,24 +429,25 @@ __device__ __forceinline__ void eval_m2p(WarpSmem& sm, int head, int cnt,
     pi = fma2(Qi, s, pi);
   }
   __syncwarp();
-  kahan_add(acc.sx, acc.cx, fx.x + fx.y);
-  kahan_add(acc.sy, acc.cy, fy.x + fy.y);
-  kahan_add(acc.sz, acc.cz, fz.x + fz.y);
-  phi_add(sm, lane, (double)pa.x + (double)pa.y, (double)pi.x + (double)pi.y);
+  out.fx = fx.x + fx.y;
+  out.fy = fy.x + fy.y;
+  out.fz = fz.x + fz.y;
+  out.pa = (double)pa.x + (double)pa.y;
+  out.pi = (double)pi.x + (double)pi.y;
 }
 
 // -------------------------------------------------------------- local ----
 // Up to 32 far cells, one per lane: each lane expands its cell's field about
 // the group centre G (local.cuh) into its row of `loc_rows`; lanes 0..28 then
-// add one coefficient each over the rows to their running sum `lsum`.  The
+// add up one coefficient each over the rows.  The
 // group's targets evaluate the summed expansion once, after the walk.
 template <int ORDER>
-__device__ __forceinline__ void eval_local(WarpSmem& sm, int head, int cnt,
+__device__ __forceinline__ void eval_local(WarpSmem& sm, const int* list, int mask, int head, int cnt,
                                            const MixedArgs& a, double Gx, double Gy,
-                                           double Gz, int lane, float& lsum) {
+                                           double Gz, int lane, Batch& out) {
   constexpr int kStride = kLocStride;
   if (lane < cnt) {
-    const int node = sm.loc[(head + lane) & (kLocRing - 1)];
+    const int node = list[(head + lane) & mask];
     const double4 c = ldg_d4(&a.node_c[node]);
     CellMoments m;
     const float4* mp = a.mom + 3 * (int64_t)node;
@@ -437,11 +475,10 @@ __device__ __forceinline__ void eval_local(WarpSmem& sm, int head, int cnt,
                        sm.loc_rows + kStride * lane);
   }
   __syncwarp();
-  if (lane < kLocCoef) {
-    float t = 0.f;
+  float t = 0.f;
+  if (lane < kLocCoef)
     for (int k = 0; k < cnt; ++k) t += sm.loc_rows[kStride * k + lane];
-    lsum += t;
-  }
+  out.loc = t;
   __syncwarp();
 }
 
@@ -563,18 +600,18 @@ __device__ __forceinline__ void p2p_one(const WarpSmem& sm, float r2, float dx, 
 // Coulomb from the hi parts; a close pair (r^2 <= close2) is redone with the
 // exact offsets, and a pair with a special member goes through p2p_one.
 template <int PHYS, bool RDF>
-__device__ __forceinline__ void eval_p2p(WarpSmem& sm, int head, int cnt,
+__device__ __forceinline__ void eval_p2p(WarpSmem& sm, const int* list, int cnt,
                                          const MixedArgs& a, double Gx,
                                          double Gy, double Gz, float thx,
                                          float thy, float thz, float tlx,
                                          float tly, float tlz, float close2,
                                          int p_self, int tsp, bool act, int lane,
-                                         uint32_t* hist, Acc& acc) {
+                                         uint32_t* hist, Batch& out) {
   {
     // this lane's source (or, past cnt, a chargeless dummy beyond any RDF bin)
     float v[8];
     if (lane < cnt) {
-      const int s = sm.p2p[head + lane];
+      const int s = list[lane];
       const double4 xs = a.xs[s];
       const double rx = Gx - xs.x, ry = Gy - xs.y, rz = Gz - xs.z;
       const float hx = (float)rx, hy = (float)ry, hz = (float)rz;
@@ -694,11 +731,12 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, int head, int cnt,
     if (RDF && act) rdf_count2<PHYS>(a, hist, r2, rinv, q, s0, s1, p_self, tsp);
   }
   __syncwarp();
-  kahan_add(acc.sx, acc.cx, fx.x + fx.y);
-  kahan_add(acc.sy, acc.cy, fy.x + fy.y);
-  kahan_add(acc.sz, acc.cz, fz.x + fz.y);
+  out.fx = fx.x + fx.y;
+  out.fy = fy.x + fy.y;
+  out.fz = fz.x + fz.y;
   const double pad = (double)pa.x + (double)pa.y, pqd = (double)pq.x + (double)pq.y;
-  phi_add(sm, lane, pad, 0.5 * (pad + pqd));  // ion sources: (all + charge-weighted) / 2
+  out.pa = pad;
+  out.pi = 0.5 * (pad + pqd);  // ion sources: (all + charge-weighted) / 2
 }
 
 // Squared distance from a cell's centroid to the group's box, in an
@@ -790,11 +828,18 @@ constexpr size_t walk_smem_bytes(int warps) {
   return sizeof(WarpSmem) * warps + walk_learned_bytes<LEARNED, RDF>() +
          (RDF ? sizeof(uint32_t) * 2 * kRdfBins : 0);
 }
+constexpr size_t kTeamBytes = sizeof(TeamSmem) * (16 / kTeamMin);
+static_assert(walk_smem_bytes<true, true>(16) + kTeamBytes <= 227 * 1024, "team walk over 227 KB");
 static_assert(walk_smem_bytes<true, true>(16) <= 195 * 1024, "RDF walk over the 196 KB step");
 static_assert(walk_smem_bytes<false, false>(20) <= 163 * 1024, "walk over the 164 KB step");
 
-template <int PHYS, bool RDF, bool LEARNED, int ORDER>
-__global__ void __launch_bounds__(32 * walk_warps<RDF, LEARNED>(), 1) k_walk_mixed(MixedArgs a) {
+__device__ __forceinline__ void team_sync(int team, int warps) {
+  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * warps) : "memory");
+}
+
+template <int PHYS, bool RDF, bool LEARNED, int ORDER, bool TEAM>
+__global__ void __launch_bounds__(32 * (TEAM ? 16 : walk_warps<RDF, LEARNED>()), 1)
+    k_walk_mixed(MixedArgs a) {
   extern __shared__ float4 dyn_smem[];
   WarpSmem* smem = reinterpret_cast<WarpSmem*>(dyn_smem);
   const int nwarps = blockDim.x >> 5;
@@ -809,6 +854,11 @@ __global__ void __launch_bounds__(32 * walk_warps<RDF, LEARNED>(), 1) k_walk_mix
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   WarpSmem& sm = smem[wib];
+  // this warp's team, and its rank in it (0: the leader)
+  const int team = TEAM ? wib / a.team : wib, rank = TEAM ? wib & (a.team - 1) : 0;
+  const int nteams = TEAM ? nwarps / a.team : nwarps;
+  TeamSmem& ts = reinterpret_cast<TeamSmem*>(
+      tail + walk_learned_bytes<LEARNED, RDF>() + (RDF ? sizeof(uint32_t) * 2 * kRdfBins : 0))[team];
   if (RDF) {
     for (int i = threadIdx.x; i < 2 * kRdfBins; i += blockDim.x) hist[i] = 0u;
     __syncthreads();
@@ -837,11 +887,18 @@ __global__ void __launch_bounds__(32 * walk_warps<RDF, LEARNED>(), 1) k_walk_mix
   // The first group of each warp is fixed, spread over the SMs before the warps
   // of an SM: with fewer groups than warps, a cursor alone gives them all to
   // the blocks that start first (N = 32,768 kept 55 of the 148 SMs busy).
-  int g = wib * gridDim.x + blockIdx.x;
+  int g = team * gridDim.x + blockIdx.x;
   for (bool own = true; root_end > 0; own = false) {
     if (!own) {
-      if (lane == 0) g = gridDim.x * nwarps + atomicAdd(&a.control[0], 1);
-      g = __shfl_sync(0xffffffffu, g, 0);
+      if (lane == 0 && rank == 0) g = gridDim.x * nteams + atomicAdd(&a.control[0], 1);
+      if (TEAM) {
+        if (lane == 0 && rank == 0) ts.item = g;
+        __syncwarp();
+        team_sync(team, a.team);
+        g = ts.item;
+      } else {
+        g = __shfl_sync(0xffffffffu, g, 0);
+      }
     }
     if (g >= ngroups) break;
     const int2 grp = a.groups[g];
@@ -922,160 +979,217 @@ __global__ void __launch_bounds__(32 * walk_warps<RDF, LEARNED>(), 1) k_walk_mix
     bool overflow = false;
     int cqh = 0, cqt = 0;  // learned-MAC candidate ring (warp-uniform)
     bool fin = false;
-    while (!fin) {
-      int node = -1;
-      int action = 0, pfirst = 0, pcnt = 0;  // 1 far field, 2 particles, 3 open
-      if (LEARNED && (cqt - cqh >= 32 || (ssize == 0 && cqt > cqh))) {
-        // ---- a batch of queued candidates goes through the network ----
-        const int nb = min(32, cqt - cqh);
-        const bool cand = lane < nb;
-        if (cand) node = sm.cq_node[(cqh + lane) & (kCandRing - 1)];
-        cqh += nb;
-        __syncwarp();
-        const int r = mac_batch(a.node_c, a.geom, a.mom, a.mom3, sm, mlp, frange, node, cand,
-                                (float)n_act, lane);
-        if (cand) action = r & 3;  // candidates exceed a bucket: accept or open
-        const unsigned fbm = __ballot_sync(0xffffffffu, (r & 4) != 0);
-        if (lane == 0) {
-          sm.n_mlp += (unsigned)nb;
-          sm.n_fallback += (unsigned)__popc(fbm);
-        }
-      } else {
-        // ---- a batch of nodes from the stack ----
-        const int nb = min(32, ssize);
-        node = lane < nb ? stack[ssize - 1 - lane] : -1;
-        ssize -= nb;
-        __syncwarp();
-        bool cand = false;  // queued for the learned MAC
-        if (node >= 0) {
-          // the particle range and (learned criterion) the cell's pre-filter
-          // record depend on the node index alone: issued with node_c, so a
-          // batch waits for one round of loads instead of two or three
-          const double4 c = ldg_d4(&a.node_c[node]);
-          const int cnt = __ldg(&a.count[node]);
-          const int fst = __ldg(&a.first[node]);
-          const float2 kr = LEARNED ? __ldg(&a.mac_k[node]) : make_float2(0.f, 0.f);
-          if (c.w < 0.0) {
-            action = 2;
-            pfirst = fst;
-            pcnt = 1;
-          } else {
-            // group MAC: rcrit below the distance from the centroid to the box
-            const double d2 = box_dist2(c, sm);
-            bool accept = c.w * c.w < d2;  // the fixed-theta test
-            if (LEARNED && !accept) {
-              // learned criterion, on top of the fixed test: a cell the fixed
-              // test opens is accepted anyway when its predicted acceptance
-              // error is within the group's budget.  rho = s / (d - dx) places
-              // it against the training band; est is the fitted log-linear
-              // estimate of the label (mac.cuh) and B the budget in the same
-              // units.  Cells whose estimate is clearly on one side of B
-              // (training quantiles m_lo, m_hi of label - est) are decided at
-              // once; the rest are queued for the network.  Only cells that
-              // would otherwise open into more than a bucket of particle
-              // pairs are worth a far-field evaluation.
-              // rho = s / (d - dx) <= rho_hi  <=>  d >= s / rho_hi + dx
-              const float d2f = (float)d2;
-              if (d2f >= kr.y * kr.y && cnt > a.bucket) {
-                const float ddf = sqrtf(d2f);
-                // est - B = K - log10(budget) - (2 + c0) log10(d); no
-                // budget: log10(budget) = -inf, never accepted or queued
-                const float lb = sm.lbud, l10d = __log10f(ddf);
-                const float eb = fmaf(-(2.f + fmodel[2]), l10d, kr.x - lb);
-                if (eb + fmodel[1] <= 0.f) {
-                  accept = true;
-                } else if (eb + fmodel[0] <= 0.f) {
-                  cand = true;
-                }
-              }
-            }
-            // a small accepted cell is cheaper and exact as particle pairs: an
-            // M2P costs about as much as p2p_max pair interactions
-            if (accept && cnt <= a.p2p_max) {
+    int qn = 0;  // TEAM: batches in the queue
+    while (TEAM || !fin) {
+      // ---- a batch of nodes (TEAM: until a round's worth of work waits) ----
+      while (rank == 0 && !fin && (!TEAM || qn < a.team)) {
+        int node = -1;
+        int action = 0, pfirst = 0, pcnt = 0;  // 1 far field, 2 particles, 3 open
+        if (LEARNED && (cqt - cqh >= 32 || (ssize == 0 && cqt > cqh))) {
+          // ---- a batch of queued candidates goes through the network ----
+          const int nb = min(32, cqt - cqh);
+          const bool cand = lane < nb;
+          if (cand) node = sm.cq_node[(cqh + lane) & (kCandRing - 1)];
+          cqh += nb;
+          __syncwarp();
+          const int r = mac_batch(a.node_c, a.geom, a.mom, a.mom3, sm, mlp, frange, node, cand,
+                                  (float)n_act, lane);
+          if (cand) action = r & 3;  // candidates exceed a bucket: accept or open
+          const unsigned fbm = __ballot_sync(0xffffffffu, (r & 4) != 0);
+          if (lane == 0) {
+            sm.n_mlp += (unsigned)nb;
+            sm.n_fallback += (unsigned)__popc(fbm);
+          }
+        } else {
+          // ---- a batch of nodes from the stack ----
+          const int nb = min(32, ssize);
+          node = lane < nb ? stack[ssize - 1 - lane] : -1;
+          ssize -= nb;
+          __syncwarp();
+          bool cand = false;  // queued for the learned MAC
+          if (node >= 0) {
+            // the particle range and (learned criterion) the cell's pre-filter
+            // record depend on the node index alone: issued with node_c, so a
+            // batch waits for one round of loads instead of two or three
+            const double4 c = ldg_d4(&a.node_c[node]);
+            const int cnt = __ldg(&a.count[node]);
+            const int fst = __ldg(&a.first[node]);
+            const float2 kr = LEARNED ? __ldg(&a.mac_k[node]) : make_float2(0.f, 0.f);
+            if (c.w < 0.0) {
               action = 2;
               pfirst = fst;
-              pcnt = cnt;
-            } else if (accept) {
-              action = 1;
-              if (a.loc_eps2 > 0.0) {
-                // far from the group: summed into its local expansion
-                const double ux = c.x - sm.gx, uy = c.y - sm.gy, uz = c.z - sm.gz;
-                const double dc2 = ux * ux + uy * uy + uz * uz;
-                if (sm.hl2 <= a.loc_eps2 * dc2) action = 4;
+              pcnt = 1;
+            } else {
+              // group MAC: rcrit below the distance from the centroid to the box
+              const double d2 = box_dist2(c, sm);
+              bool accept = c.w * c.w < d2;  // the fixed-theta test
+              if (LEARNED && !accept) {
+                // learned criterion, on top of the fixed test: a cell the fixed
+                // test opens is accepted anyway when its predicted acceptance
+                // error is within the group's budget.  rho = s / (d - dx) places
+                // it against the training band; est is the fitted log-linear
+                // estimate of the label (mac.cuh) and B the budget in the same
+                // units.  Cells whose estimate is clearly on one side of B
+                // (training quantiles m_lo, m_hi of label - est) are decided at
+                // once; the rest are queued for the network.  Only cells that
+                // would otherwise open into more than a bucket of particle
+                // pairs are worth a far-field evaluation.
+                // rho = s / (d - dx) <= rho_hi  <=>  d >= s / rho_hi + dx
+                const float d2f = (float)d2;
+                if (d2f >= kr.y * kr.y && cnt > a.bucket) {
+                  const float ddf = sqrtf(d2f);
+                  // est - B = K - log10(budget) - (2 + c0) log10(d); no
+                  // budget: log10(budget) = -inf, never accepted or queued
+                  const float lb = sm.lbud, l10d = __log10f(ddf);
+                  const float eb = fmaf(-(2.f + fmodel[2]), l10d, kr.x - lb);
+                  if (eb + fmodel[1] <= 0.f) {
+                    accept = true;
+                  } else if (eb + fmodel[0] <= 0.f) {
+                    cand = true;
+                  }
+                }
               }
-            } else if (!cand) {
-              if (cnt <= a.bucket) {
+              // a small accepted cell is cheaper and exact as particle pairs: an
+              // M2P costs about as much as p2p_max pair interactions
+              if (accept && cnt <= a.p2p_max) {
                 action = 2;
                 pfirst = fst;
                 pcnt = cnt;
-              } else {
-                action = 3;
+              } else if (accept) {
+                action = 1;
+                if (a.loc_eps2 > 0.0) {
+                  // far from the group: summed into its local expansion
+                  const double ux = c.x - sm.gx, uy = c.y - sm.gy, uz = c.z - sm.gz;
+                  const double dc2 = ux * ux + uy * uy + uz * uz;
+                  if (sm.hl2 <= a.loc_eps2 * dc2) action = 4;
+                }
+              } else if (!cand) {
+                if (cnt <= a.bucket) {
+                  action = 2;
+                  pfirst = fst;
+                  pcnt = cnt;
+                } else {
+                  action = 3;
+                }
               }
             }
           }
-        }
-        if (LEARNED) {
-          const unsigned cm = __ballot_sync(0xffffffffu, cand);
-          if (cand) {
-            const int q = (cqt + __popc(cm & lt)) & (kCandRing - 1);
-            sm.cq_node[q] = node;
+          if (LEARNED) {
+            const unsigned cm = __ballot_sync(0xffffffffu, cand);
+            if (cand) {
+              const int q = (cqt + __popc(cm & lt)) & (kCandRing - 1);
+              sm.cq_node[q] = node;
+            }
+            cqt += __popc(cm);
           }
-          cqt += __popc(cm);
+        }
+        // far-field entries
+        const unsigned bm = __ballot_sync(0xffffffffu, action == 1);
+        if (action == 1) sm.m2p[(m2t + __popc(bm & lt)) & (kM2pRing - 1)] = node;
+        m2t += __popc(bm);
+        // local-expansion entries
+        const unsigned lm = __ballot_sync(0xffffffffu, action == 4);
+        if (action == 4) sm.loc[(lct + __popc(lm & lt)) & (kLocRing - 1)] = node;
+        lct += __popc(lm);
+        // particle entries
+        int ptot;
+        const int pex = warp_excl_scan(action == 2 ? pcnt : 0, lane, &ptot);
+        if (action == 2)
+          for (int k = 0; k < pcnt; ++k)
+            sm.p2p[p2n + pex + k] = pfirst + k;
+        p2n += ptot;
+        // opened twigs push their children (octant order)
+        int4 k0 = make_int4(-1, -1, -1, -1), k1 = k0;
+        if (action == 3) {
+          const int4* kk = reinterpret_cast<const int4*>(a.kids + 8 * (int64_t)node);
+          k0 = __ldg(kk);
+          k1 = __ldg(kk + 1);
+        }
+        const int kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+        int kc = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) kc += kv[j] >= 0 ? 1 : 0;
+        int ktot;
+        const int kex = warp_excl_scan(kc, lane, &ktot);
+        if (ssize + ktot > kStackCap) {
+          overflow = fin = true;
+          qn = 0;
+          break;
+        }
+        {
+          int pos = ssize + kex;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (kv[j] >= 0) stack[pos++] = kv[j];
+        }
+        ssize += ktot;
+        max_stack = max(max_stack, ssize);
+        __syncwarp();
+        fin = ssize == 0 && cqt == cqh;
+        if (!TEAM) break;
+        // full batches, and what is left once the walk has ended, to the queue
+        int p2h = 0;
+        while (p2n - p2h >= 32 || (fin && p2n > p2h)) {
+          const int cnt = min(32, p2n - p2h);
+          if (lane < cnt) ts.idx[qn][lane] = sm.p2p[p2h + lane];
+          if (lane == 0) ts.info[qn] = 4 * cnt + 2;
+          ++qn;
+          p2h += cnt;
+        }
+        p2tot += p2h;
+        p2n -= p2h;
+        if (p2h > 0) {  // the remainder moves to the front
+          const int e = lane < p2n ? sm.p2p[p2h + lane] : 0;
+          __syncwarp();
+          if (lane < p2n) sm.p2p[lane] = e;
+        }
+        while (m2t - m2h >= 32 || (fin && m2t > m2h)) {
+          const int cnt = min(32, m2t - m2h);
+          if (lane < cnt) ts.idx[qn][lane] = sm.m2p[(m2h + lane) & (kM2pRing - 1)];
+          if (lane == 0) ts.info[qn] = 4 * cnt + 1;
+          ++qn;
+          m2h += cnt;
+        }
+        while (lct - lch >= 32 || (fin && lct > lch)) {
+          const int cnt = min(32, lct - lch);
+          if (lane < cnt) ts.idx[qn][lane] = sm.loc[(lch + lane) & (kLocRing - 1)];
+          if (lane == 0) ts.info[qn] = 4 * cnt + 3;
+          ++qn;
+          lch += cnt;
+        }
+        __syncwarp();
+      }
+      // ---- evaluation: full batches of 32, and what is left once the walk has
+      // ended.  One call site each: this is long straight-line code, and the
+      // warps of an SM are in different parts of it. ----
+      if (!TEAM && overflow) break;
+      int take = 0, kind = 0, cnt = 0;
+      Batch out;
+      if (TEAM) out = {0.f, 0.f, 0.f, 0.f, 0.0, 0.0};
+      int p2h = 0;
+      if (TEAM) {
+        if (rank == 0) {
+          take = min(qn, a.team);
+          if (lane == 0) ts.take = take;
+        }
+        __syncwarp();
+        team_sync(team, a.team);
+        take = ts.take;
+        if (take == 0) break;
+        if (rank < take) {
+          kind = ts.info[rank] & 3;
+          cnt = ts.info[rank] >> 2;
         }
       }
-      // far-field entries
-      const unsigned bm = __ballot_sync(0xffffffffu, action == 1);
-      if (action == 1) sm.m2p[(m2t + __popc(bm & lt)) & (kM2pRing - 1)] = node;
-      m2t += __popc(bm);
-      // local-expansion entries
-      const unsigned lm = __ballot_sync(0xffffffffu, action == 4);
-      if (action == 4) sm.loc[(lct + __popc(lm & lt)) & (kLocRing - 1)] = node;
-      lct += __popc(lm);
-      // particle entries
-      int ptot;
-      const int pex = warp_excl_scan(action == 2 ? pcnt : 0, lane, &ptot);
-      if (action == 2)
-        for (int k = 0; k < pcnt; ++k)
-          sm.p2p[p2n + pex + k] = pfirst + k;
-      p2n += ptot;
-      // opened twigs push their children (octant order)
-      int4 k0 = make_int4(-1, -1, -1, -1), k1 = k0;
-      if (action == 3) {
-        const int4* kk = reinterpret_cast<const int4*>(a.kids + 8 * (int64_t)node);
-        k0 = __ldg(kk);
-        k1 = __ldg(kk + 1);
-      }
-      const int kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-      int kc = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) kc += kv[j] >= 0 ? 1 : 0;
-      int ktot;
-      const int kex = warp_excl_scan(kc, lane, &ktot);
-      if (ssize + ktot > kStackCap) {
-        overflow = true;
-        break;
-      }
-      {
-        int pos = ssize + kex;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (kv[j] >= 0) stack[pos++] = kv[j];
-      }
-      ssize += ktot;
-      max_stack = max(max_stack, ssize);
-      __syncwarp();
-      // Full batches of 32, and what is left once the walk has ended.  One
-      // call site each: the evaluations are long straight-line code, and the
-      // warps of an SM are in different ones.
-      fin = ssize == 0 && cqt == cqh;
-      int p2h = 0;
-      while (p2n - p2h >= 32 || (fin && p2n > p2h)) {
-        const int cnt = min(32, p2n - p2h);
-        eval_p2p<PHYS, RDF>(sm, p2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, tlx, tly, tlz,
-                            close2, pt, tsp, act, lane, hist, acc);
+      while (TEAM ? kind == 2 : p2n - p2h >= 32 || (fin && p2n > p2h)) {
+        if (!TEAM) cnt = min(32, p2n - p2h);
+        eval_p2p<PHYS, RDF>(sm, TEAM ? ts.idx[rank] : sm.p2p + p2h, cnt, a, sm.gx, sm.gy, sm.gz,
+                            thx, thy, thz, tlx, tly, tlz, close2, pt, tsp, act, lane, hist, out);
+        if (TEAM) break;
+        batch_add(sm, lane, acc, out);
         p2h += cnt;
       }
-      if (p2h > 0) {  // the remainder moves to the front
+      if (!TEAM && p2h > 0) {  // the remainder moves to the front
         p2tot += p2h;
         p2n -= p2h;
         const int e = lane < p2n ? sm.p2p[p2h + lane] : 0;
@@ -1083,17 +1197,45 @@ __global__ void __launch_bounds__(32 * walk_warps<RDF, LEARNED>(), 1) k_walk_mix
         if (lane < p2n) sm.p2p[lane] = e;
         __syncwarp();
       }
-      while (m2t - m2h >= 32 || (fin && m2t > m2h)) {
-        const int cnt = min(32, m2t - m2h);
-        eval_m2p<ORDER>(sm, m2h, cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, acc);
+      while (TEAM ? kind == 1 : m2t - m2h >= 32 || (fin && m2t > m2h)) {
+        if (!TEAM) cnt = min(32, m2t - m2h);
+        eval_m2p<ORDER>(sm, TEAM ? ts.idx[rank] : sm.m2p, TEAM ? 31 : kM2pRing - 1, TEAM ? 0 : m2h,
+                        cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, out);
+        if (TEAM) break;
+        batch_add(sm, lane, acc, out);
         m2h += cnt;
       }
-      while (lct - lch >= 32 || (fin && lct > lch)) {
-        const int cnt = min(32, lct - lch);
-        eval_local<ORDER>(sm, lch, cnt, a, sm.gx, sm.gy, sm.gz, lane, lsum);
+      while (TEAM ? kind == 3 : lct - lch >= 32 || (fin && lct > lch)) {
+        if (!TEAM) cnt = min(32, lct - lch);
+        eval_local<ORDER>(sm, TEAM ? ts.idx[rank] : sm.loc, TEAM ? 31 : kLocRing - 1,
+                          TEAM ? 0 : lch, cnt, a, sm.gx, sm.gy, sm.gz, lane, out);
+        if (TEAM) break;
+        lsum += out.loc;
         lch += cnt;
       }
+      if (TEAM) {
+        // results stay in each warp's staging buffer until the leader has them
+        if (rank < take) reinterpret_cast<Batch*>(sm.cell)[lane] = out;
+        __syncwarp();
+        team_sync(team, a.team);
+        if (rank == 0) {
+          for (int j = 0; j < take; ++j) {
+            const Batch b = reinterpret_cast<const Batch*>(smem[wib + j].cell)[lane];
+            if ((ts.info[j] & 3) == 3) lsum += b.loc;
+            else batch_add(sm, lane, acc, b);
+          }
+          qn -= take;
+          for (int j = 0; j < qn; ++j) {  // what is left of the queue moves up
+            const int e = ts.idx[j + take][lane], f = ts.info[j + take];
+            __syncwarp();
+            ts.idx[j][lane] = e;
+            if (lane == 0) ts.info[j] = f;
+            __syncwarp();
+          }
+        }
+      }
     }
+    if (TEAM && rank != 0) continue;
     if (overflow) {
       if (lane == 0) set_error(a.err, kErrWalk);
       continue;
@@ -1292,30 +1434,36 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
   // holds (a fixed 16 with RDF counts)
   const int bps = tune.blocks_per_sm < 1 ? 1 : (tune.blocks_per_sm > kMaxBlocksPerSm ? kMaxBlocksPerSm : tune.blocks_per_sm);
   const bool r = rdf != nullptr;
+  a.team = walk_team(n);
   if (L) k_mac_node_terms<<<mb.sms * 4, 256, 0, st>>>(mb.geom, mb.mom3, tv.tree_bounds,
                                                        learned->margins, 1.f / learned->rho_hi,
                                                        mb.mac_k);
   int dev = 0;
   cudaGetDevice(&dev);
-#define TG_LAUNCH(P, R, LL, O)                                                \
+#define TG_LAUNCH(P, R, LL, O, S)                                             \
   do {                                                                        \
-    auto kfn = k_walk_mixed<P, R, LL, O>;                                     \
-    const int most = walk_warps<R, LL>();                                     \
-    const int nw = R || kWarpStep * bps > most ? most : kWarpStep * bps;      \
-    const size_t sb = walk_smem_bytes<LL, R>(nw);                             \
+    auto kfn = k_walk_mixed<P, R, LL, O, S>;                                  \
+    const int most = S ? 16 : walk_warps<R, LL>();                            \
+    const int nw = S || R || kWarpStep * bps > most ? most : kWarpStep * bps; \
+    const size_t sb = walk_smem_bytes<LL, R>(nw) + (S ? kTeamBytes : 0);      \
     static unsigned attr_set = 0; /* devices with the smem limit raised */    \
     if (dev < 32 && !(attr_set & (1u << dev))) {                              \
       cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                           (int)walk_smem_bytes<LL, R>(most));                \
+                           (int)(walk_smem_bytes<LL, R>(most) + (S ? kTeamBytes : 0))); \
       attr_set |= 1u << dev;                                                  \
     }                                                                         \
     kfn<<<mb.sms, 32 * nw, sb, st>>>(a);                                      \
   } while (0)
 #define TG_LAUNCH_O(P, R, LL)                                                 \
   do {                                                                        \
-    if (tune.order >= 4) TG_LAUNCH(P, R, LL, 4);                              \
-    else if (tune.order == 3) TG_LAUNCH(P, R, LL, 3);                         \
-    else TG_LAUNCH(P, R, LL, 2);                                              \
+    if (a.team > 1) TG_LAUNCH_S(P, R, LL, true);                              \
+    else TG_LAUNCH_S(P, R, LL, false);                                        \
+  } while (0)
+#define TG_LAUNCH_S(P, R, LL, S)                                              \
+  do {                                                                        \
+    if (tune.order >= 4) TG_LAUNCH(P, R, LL, 4, S);                           \
+    else if (tune.order == 3) TG_LAUNCH(P, R, LL, 3, S);                      \
+    else TG_LAUNCH(P, R, LL, 2, S);                                           \
   } while (0)
   if (wp.physics == 1) {
     if (L) { if (r) TG_LAUNCH_O(1, true, true); else TG_LAUNCH_O(1, false, true); }
@@ -1325,6 +1473,7 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
     else { if (r) TG_LAUNCH_O(0, true, false); else TG_LAUNCH_O(0, false, false); }
   }
 #undef TG_LAUNCH_O
+#undef TG_LAUNCH_S
 #undef TG_LAUNCH
   return L ? 2 : 1;
 }
