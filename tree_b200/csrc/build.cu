@@ -46,9 +46,10 @@ __device__ __forceinline__ uint64_t shfl_max_u64(uint64_t v) {
   return v;
 }
 
-// bb[(s*3+k)*2 + 0] = ord(min), +1 = ord(max)
-__global__ void k_bbox(const double* __restrict__ x, int n, int n_el,
-                       uint64_t* bb, int32_t* err) {
+// bb[(s*3+k)*2 + 0] = ord(min), +1 = ord(max) over the particles first,
+// first + stride, ... of each species
+__device__ __forceinline__ void bbox_of(const double* __restrict__ x, int n, int n_el, int first,
+                                        int stride, uint64_t* bb, int32_t* err) {
   uint64_t mn[2][3], mx[2][3];
 #pragma unroll
   for (int s = 0; s < 2; ++s)
@@ -58,8 +59,7 @@ __global__ void k_bbox(const double* __restrict__ x, int n, int n_el,
       mx[s][k] = 0ull;
     }
   bool bad = false;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x) {
+  for (int i = first; i < n; i += stride) {
     int s = i >= n_el;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -89,18 +89,21 @@ __global__ void k_bbox(const double* __restrict__ x, int n, int n_el,
     }
 }
 
+__global__ void k_bbox(const double* __restrict__ x, int n, int n_el,
+                       uint64_t* bb, int32_t* err) {
+  bbox_of(x, n, n_el, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, bb, err);
+}
+
 // Root box per species: tree.f90:58-63 (xx = (max+min)/2, lx = max-min).
-__global__ void k_geom(const uint64_t* bb, int n, int n_el, Geom* g) {
-  int s = threadIdx.x;
-  if (s >= 2) return;
+__device__ __forceinline__ void geom_of(const uint64_t* bb, int n, int n_el, int s, Geom* g) {
   Geom G;
   G.n = s == 0 ? n_el : n - n_el;
   G.first = s == 0 ? 0 : n_el;
   double smax = 0.0;
   for (int k = 0; k < 3; ++k) {
     if (G.n > 0) {
-      double lo = double_from_ord(bb[(s * 3 + k) * 2]);
-      double hi = double_from_ord(bb[(s * 3 + k) * 2 + 1]);
+      double lo = double_from_ord(__ldcg((const unsigned long long*)&bb[(s * 3 + k) * 2]));
+      double hi = double_from_ord(__ldcg((const unsigned long long*)&bb[(s * 3 + k) * 2 + 1]));
       G.c0[k] = (hi + lo) / 2.0;
       G.lx0[k] = hi - lo;
     } else {
@@ -111,6 +114,10 @@ __global__ void k_geom(const uint64_t* bb, int n, int n_el, Geom* g) {
   }
   G.smax0 = smax;
   g[s] = G;
+}
+
+__global__ void k_geom(const uint64_t* bb, int n, int n_el, Geom* g) {
+  if (threadIdx.x < 2) geom_of(bb, n, n_el, threadIdx.x, g);
 }
 
 // Per-cloud bounding boxes: one block per cloud, bb[(c*3+k)*2 + 0/1] = ord
@@ -608,27 +615,25 @@ __device__ __forceinline__ int clz128(key128 x) {
 // L[p] = number of leading levels that sorted keys p and p+1 share (same
 // species tree / same cloud: equal `top` bits), else -1.  Identical keys mean
 // the level cap was hit.
+__device__ __forceinline__ int8_t common_level(key128 a, key128 b, int top, int nlev,
+                                               int32_t* err) {
+  const key128 x = a ^ b;
+  if (top > 0 && (x >> (128 - top)) != 0) return -1;
+  if (x == 0) {
+    set_error(err, kErrDepth);
+    return (int8_t)nlev;
+  }
+  // lz >= top (same tree); for the combined layouts lz = 127 means only
+  // the species bit differs, i.e. all nlev spatial levels are shared
+  const int lev = (clz128(x) - top) / 3;
+  return (int8_t)(lev < nlev ? lev : nlev);
+}
+
 __global__ void k_common_levels(const key128* __restrict__ keys, int n,
                                 int top, int nlev, int8_t* L, int32_t* err) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  int8_t r = -1;
-  if (p + 1 < n) {
-    key128 a = keys[p], b = keys[p + 1];
-    key128 x = a ^ b;
-    if (top == 0 || (x >> (128 - top)) == 0) {
-      if (x == 0) {
-        set_error(err, kErrDepth);
-        r = (int8_t)nlev;
-      } else {
-        // lz >= top (same tree); for the combined layouts lz = 127 means only
-        // the species bit differs, i.e. all nlev spatial levels are shared
-        int lev = (clz128(x) - top) / 3;
-        r = (int8_t)(lev < nlev ? lev : nlev);
-      }
-    }
-  }
-  L[p] = r;
+  L[p] = p + 1 < n ? common_level(keys[p], keys[p + 1], top, nlev, err) : (int8_t)-1;
 }
 
 __global__ void k_counts(const int8_t* __restrict__ L, int n, int32_t* cnt) {
@@ -943,19 +948,159 @@ __global__ void k_roots(const int32_t* __restrict__ off,
   if (c < nseg) roots[c] = off[start[c]];
 }
 
+// me, m: nodes of the first tree, of both.
+__device__ __forceinline__ void write_bounds(int me, int m, int cap, int32_t* bounds,
+                                             int32_t* err) {
+  if (m > cap) set_error(err, kErrCapacity);
+  bounds[0] = 0;
+  bounds[1] = me < cap ? me : cap;
+  bounds[2] = m < cap ? m : cap;
+  bounds[3] = m;  // untruncated node count (for capacity growth)
+}
+
 __global__ void k_bounds(const int32_t* __restrict__ off, int n, int n_el,
                          int cap, int32_t* bounds, int32_t* err) {
-  if (threadIdx.x != 0) return;
-  int me = off[n_el], m = off[n];
-  if (m > cap) {
-    set_error(err, kErrCapacity);
-    me = me < cap ? me : cap;
-    m = cap;
+  if (threadIdx.x == 0) write_bounds(off[n_el], off[n], cap, bounds, err);
+}
+
+// ------------------------------------------------ front of a small build ----
+// Up to kFrontMax particles two launches do what takes 50 above (the radix
+// sort's 40 among them): a small build is a chain of launches, 2.5 to 4 us each
+// in a step graph, on arrays that hardly fill one SM.  With k_bbox_small,
+// k_net_small and k_groups_small a build takes (us in the step graph, mixed |
+// FP64 path):
+//   N = 1,000   194 -> 56  | 199 -> 70
+//   N = 4,000   254 -> 96  | 237 -> 92
+//   N = 8,192   271 -> 147 | 257 -> 130
+//   N = 16,384  317 -> 303 | 273 -> 248, where the n^2 comparisons catch up.
+constexpr int kFrontThreads = 1024;
+constexpr int kFrontItems = 16;
+constexpr int kFrontMax = kFrontThreads * kFrontItems;
+
+// Sorts by counting: the rank of a key is the number of keys below it (equal
+// full keys keep their order), n^2 comparisons spread over all SMs: 7 us at
+// 1,000 keys, 16 us at 4,096.  A block ranks 32 keys, one per lane; each of
+// its 16 warps compares them with 1/16 of every tile of keys.
+constexpr int kRankWarps = 16;
+constexpr int kRankTile = 1024;
+__global__ void __launch_bounds__(32 * kRankWarps)
+    k_rank(const key128* __restrict__ keys_in, int n, key128* __restrict__ keys,
+           uint32_t* __restrict__ vals) {
+  __shared__ uint64_t hi[kRankTile], lo[kRankTile];
+  __shared__ int32_t part[kRankWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  const key128 key = i < n ? keys_in[i] : 0;
+  const uint64_t kh = (uint64_t)(key >> 64), kl = (uint64_t)key;
+  int below = 0;
+  for (int base = 0; base < n; base += kRankTile) {
+    __syncthreads();
+    for (int j = threadIdx.x; j < kRankTile && base + j < n; j += blockDim.x) {
+      const key128 k = keys_in[base + j];
+      hi[j] = (uint64_t)(k >> 64);
+      lo[j] = (uint64_t)k;
+    }
+    __syncthreads();
+    const int m = n - base < kRankTile ? n - base : kRankTile;
+    constexpr int kSpan = kRankTile / kRankWarps;
+    const int j1 = (w + 1) * kSpan < m ? (w + 1) * kSpan : m;
+#pragma unroll 8
+    for (int j = w * kSpan; j < j1; ++j) {
+      const uint64_t h = hi[j];
+      bool lt = h < kh;
+      if (h == kh) lt = lo[j] < kl || (lo[j] == kl && base + j < i);
+      below += lt ? 1 : 0;
+    }
   }
-  bounds[0] = 0;
-  bounds[1] = me;
-  bounds[2] = m;
-  bounds[3] = off[n];  // untruncated node count (for capacity growth)
+  part[w][lane] = below;
+  __syncthreads();
+  if (w == 0 && i < n) {
+    int r = 0;
+#pragma unroll
+    for (int k = 0; k < kRankWarps; ++k) r += part[k][lane];
+    keys[r] = key;
+    vals[r] = (uint32_t)i;
+  }
+}
+
+// What follows the sort, in one block: k_common_levels, k_counts, the scan,
+// k_bounds, (owner != nullptr) k_owner, and the zero of *climbs (k_net_small's
+// list of climb starts).
+struct FrontSmem {
+  int8_t L[kFrontMax];
+  int32_t wsum[kFrontThreads / 32];
+  int32_t me;
+};
+
+__global__ void __launch_bounds__(kFrontThreads)
+    k_front(const key128* __restrict__ keys, int n, int split, int top, int nlev, int cap,
+            int8_t* L, int32_t* off, int32_t* owner, int32_t* bounds, int32_t* climbs,
+            int32_t* err) {
+  __shared__ FrontSmem s;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int iters = (n + kFrontThreads - 1) / kFrontThreads;
+  for (int p = threadIdx.x; p < n; p += kFrontThreads) {
+    const int8_t r = p + 1 < n ? common_level(keys[p], keys[p + 1], top, nlev, err) : (int8_t)-1;
+    L[p] = r;
+    s.L[p] = r;
+  }
+  __syncthreads();
+  // node offsets: thread t owns particles [iters t, iters (t + 1))
+  auto count = [&](int p) {
+    int lo, hi;
+    lo_hi(s.L, p, lo, hi);
+    return (hi > lo ? hi - lo : 0) + 1;
+  };
+  const int p0 = threadIdx.x * iters, p1 = p0 + iters < n ? p0 + iters : n;
+  int32_t sum = 0;
+  for (int p = p0; p < p1; ++p) sum += count(p);
+  int32_t inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) s.wsum[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    int32_t t = s.wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t u = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += u;
+    }
+    s.wsum[lane] = t;  // inclusive over warps
+  }
+  __syncthreads();
+  int32_t o = inc - sum + (w > 0 ? s.wsum[w - 1] : 0);
+  for (int p = p0; p < p1; ++p) {
+    const int c = count(p);
+    off[p] = o;
+    if (p == split) s.me = o;
+    if (owner)
+      for (int i = o; i < o + c && i < cap; ++i) owner[i] = p;
+    o += c;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int32_t total = s.wsum[kFrontThreads / 32 - 1];
+    off[n] = total;
+    *climbs = 0;
+    write_bounds(split < n ? s.me : total, total, cap, bounds, err);
+  }
+}
+
+// Root boxes of a small build in one block: k_bbox_init, k_bbox and k_geom.
+__global__ void __launch_bounds__(kFrontThreads)
+    k_bbox_small(const double* __restrict__ x, int n, int n_el, Geom* g, uint64_t* bb,
+                 int32_t* err) {
+  if (threadIdx.x == 0) *err = 0;
+  if (threadIdx.x < 12) bb[threadIdx.x] = (threadIdx.x & 1) ? 0ull : ~0ull;
+  __syncthreads();
+  bbox_of(x, n, n_el, threadIdx.x, blockDim.x, bb, err);
+  __threadfence();  // the atomics, before this block's own reads
+  __syncthreads();
+  if (threadIdx.x < 2) geom_of(bb, n, n_el, threadIdx.x, g);
 }
 
 // ------------------------------------------------------------- upward ----
@@ -967,7 +1112,7 @@ __global__ void k_upward(const double* __restrict__ x,
                          const int32_t* __restrict__ off, int n, int n_el,
                          const Geom* __restrict__ geom, double theta, int cap, const int32_t* __restrict__ bounds,
                          double4* node_c, double2* node_m,
-                         const int32_t* __restrict__ node_skip,
+                         const int32_t* __restrict__ kids,
                          const int32_t* __restrict__ node_parent,
                          const int32_t* __restrict__ node_nchild,
                          int32_t* node_done,
@@ -1006,20 +1151,28 @@ __global__ void k_upward(const double* __restrict__ x,
     // ---- PSeudoE/PSeudoI for twig `cur` (tree.f90:465-552) ----
     double4 gc = ldcg_d4(&node_c[cur]);
     double ox0 = gc.x, ox1 = gc.y, ox2 = gc.z;
-    int end = node_skip[cur];
-    if (end > cap) end = cap;
+    // the children in octant order, which is pre-order: all loads of a round
+    // are issued together, then summed one after the other as the reference does
+    const int4* kk = reinterpret_cast<const int4*>(kids + 8 * (int64_t)cur);
+    const int4 k0 = kk[0], k1 = kk[1];
+    const int kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+    double4 cc[8];
+    double cq[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const bool in = kv[j] > cur && kv[j] < cap;
+      if (kv[j] >= 0 && kv[j] <= cur) { set_error(err, kErrWalk); return; }
+      cc[j] = in ? ldcg_d4(&node_c[kv[j]]) : make_double4(0.0, 0.0, 0.0, 0.0);
+      cq[j] = in ? __ldcg(&node_m[5 * (int64_t)kv[j]]).x : 0.0;
+    }
     double qsum = 0.0, X0 = 0.0, X1 = 0.0, X2 = 0.0;
-    int c = cur + 1;
-    while (c < end) {
-      double4 cc = ldcg_d4(&node_c[c]);
-      double q = __ldcg(&node_m[5 * (int64_t)c]).x;
-      qsum = qsum + q;
-      X0 = X0 + q * cc.x;
-      X1 = X1 + q * cc.y;
-      X2 = X2 + q * cc.z;
-      int nx = node_skip[c];
-      if (nx <= c) { set_error(err, kErrWalk); return; }
-      c = nx;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (kv[j] < 0 || kv[j] >= cap) continue;
+      qsum = qsum + cq[j];
+      X0 = X0 + cq[j] * cc[j].x;
+      X1 = X1 + cq[j] * cc[j].y;
+      X2 = X2 + cq[j] * cc[j].z;
     }
     X0 = X0 / qsum;
     X1 = X1 / qsum;
@@ -1028,11 +1181,11 @@ __global__ void k_upward(const double* __restrict__ x,
     double dx = sqrt(a0 * a0 + a1 * a1 + a2 * a2);
     double D0 = 0.0, D1 = 0.0, D2 = 0.0, Q0 = 0.0, Q1 = 0.0, Q2 = 0.0,
            QQ0 = 0.0, QQ1 = 0.0, QQ2 = 0.0;
-    c = cur + 1;
-    while (c < end) {
-      double4 cc = ldcg_d4(&node_c[c]);
-      double q = __ldcg(&node_m[5 * (int64_t)c]).x;
-      double d0 = cc.x - X0, d1 = cc.y - X1, d2 = cc.z - X2;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (kv[j] < 0 || kv[j] >= cap) continue;
+      const double q = cq[j];
+      double d0 = cc[j].x - X0, d1 = cc[j].y - X1, d2 = cc[j].z - X2;
       D0 = D0 + q * d0;
       D1 = D1 + q * d1;
       D2 = D2 + q * d2;
@@ -1042,7 +1195,6 @@ __global__ void k_upward(const double* __restrict__ x,
       QQ0 = QQ0 + q * d0 * d1;
       QQ1 = QQ1 + q * d1 * d2;
       QQ2 = QQ2 + q * d2 * d0;
-      c = node_skip[c];
     }
     // s = MAXVAL(P%lx) at this level: each axis halves exactly per level.
     int lev = node_level[cur];
@@ -1103,10 +1255,7 @@ __global__ void k_group_levels(const int32_t* __restrict__ bounds, int cap,
 
 // Per cloud: the lowest level at which siblings may be packed, stored in the
 // last slot of the cloud's histogram row (levels stay below kLevelSlots - 1).
-__global__ void k_group_cut(int32_t* glvl, int nseg) {
-  const int seg = blockIdx.x * blockDim.x + threadIdx.x;
-  if (seg >= nseg) return;
-  int32_t* h = glvl + (int64_t)seg * kLevelSlots;
+__device__ __forceinline__ void group_cut_of(int32_t* h) {
   int64_t tot = 0;
   for (int l = 0; l < kLevelSlots - 1; ++l) tot += h[l];
   int64_t run = 0;
@@ -1119,6 +1268,11 @@ __global__ void k_group_cut(int32_t* glvl, int nseg) {
     }
   }
   h[kLevelSlots - 1] = med > kGroupSlack ? med - kGroupSlack : 0;
+}
+
+__global__ void k_group_cut(int32_t* glvl, int nseg) {
+  const int seg = blockIdx.x * blockDim.x + threadIdx.x;
+  if (seg < nseg) group_cut_of(glvl + (int64_t)seg * kLevelSlots);
 }
 
 __device__ __forceinline__ void groups_of_node(int t, const int32_t* __restrict__ node_parent,
@@ -1178,28 +1332,63 @@ __global__ void k_groups(const int32_t* __restrict__ bounds, int cap,
     groups_of_node(t, node_parent, node_level, mx, ens, glvl, groups, n_groups);
 }
 
+// The three passes in one block, for a small single cloud.
+__global__ void __launch_bounds__(1024)
+    k_groups_small(const int32_t* __restrict__ bounds, int cap,
+                   const int32_t* __restrict__ node_parent,
+                   const int8_t* __restrict__ node_level, MixedNodes mx, int2* groups,
+                   int32_t* n_groups) {
+  __shared__ int32_t h[kLevelSlots];
+  __shared__ int32_t ng;
+  if (threadIdx.x < kLevelSlots) h[threadIdx.x] = 0;
+  if (threadIdx.x == 0) ng = 0;
+  __syncthreads();
+  const int m = bounds[2] < cap ? bounds[2] : cap;
+  for (int t = threadIdx.x; t < m; t += blockDim.x) {
+    const int cnt = mx.count[t];
+    const int par = node_parent[t];
+    if (cnt <= kGroupMax && (par < 0 || mx.count[par] > kGroupMax))
+      atomicAdd(&h[node_level[t]], cnt);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) group_cut_of(h);
+  __syncthreads();
+  for (int t = threadIdx.x; t < m; t += blockDim.x)
+    groups_of_node(t, node_parent, node_level, mx, Ensemble(), h, groups, &ng);
+  __syncthreads();
+  if (threadIdx.x == 0) *n_groups = ng;
+}
+
 // ------------------------------------------------------------- driver ----
 int build_trees(const BuildBuffers& b, const double* x, int n, int n_el,
                 double theta, int mode, cudaStream_t st, bool full_records) {
   // mode 0: one tree per species (parity path); mode 1: one combined tree
   const int split = mode == 0 ? n_el : n;
   const int T = 256;
-  k_bbox_init<<<1, 32, 0, st>>>(b.bbox, b.err);
   if (n == 0) {
+    k_bbox_init<<<1, 32, 0, st>>>(b.bbox, b.err);
     cudaMemsetAsync(b.bounds, 0, 4 * sizeof(int32_t), st);
     return 1;
   }
-  int launches = 1;
+  int launches = 0;
   int gb = (n + T - 1) / T;
   int gbb = gb < 4 * 148 ? gb : 4 * 148;
+  const bool small = n <= kFrontMax;
   // an ensemble of clouds only exists on the mixed path
   const Ensemble ens = mode == 1 ? b.ens : Ensemble();
   if (ens.nseg > 0) {
+    k_bbox_init<<<1, 32, 0, st>>>(b.bbox, b.err);
     k_bbox_seg<<<ens.nseg, T, 0, st>>>(x, ens.start, b.bbox, b.err);
     k_geom_seg<<<(ens.nseg + 31) / 32, 32, 0, st>>>(b.bbox, ens.start, ens.nseg, b.geom);
+    launches += 3;
+  } else if (small) {
+    k_bbox_small<<<1, kFrontThreads, 0, st>>>(x, n, split, b.geom, b.bbox, b.err);
+    launches += 1;
   } else {
+    k_bbox_init<<<1, 32, 0, st>>>(b.bbox, b.err);
     k_bbox<<<gbb, T, 0, st>>>(x, n, split, b.bbox, b.err);
     k_geom<<<1, 32, 0, st>>>(b.bbox, n, split, b.geom);
+    launches += 3;
   }
   const int lsb = mode == 0 ? 0 : 1;
   const int top = ens.nseg > 0 ? ens.top : 1 - lsb;
@@ -1207,22 +1396,35 @@ int build_trees(const BuildBuffers& b, const double* x, int n, int n_el,
   // full keys into keys_alt, their high words into the two halves of keys
   uint64_t* hi = reinterpret_cast<uint64_t*>(b.keys);
   k_keys<<<gb, T, 0, st>>>(x, n, split, lsb, n_el, b.geom, ens, b.keys_alt, hi, b.vals);
-  launches += 3;
-  // sort the high 64 bits (8 passes over 12-byte pairs), gather the full
-  // keys in that order, then order the rare ties fully;
-  // a long tie run switches on the one-block full sort (which exits otherwise)
-  launches += radix_sort(hi, b.vals, hi + n, b.vals_alt, n, b.sort_hist, b.scan_partial, st);
-  k_gather_keys<<<gb, T, 0, st>>>(b.keys_alt, b.vals, n, b.keys);
   launches += 1;
-  cudaMemsetAsync(b.bounds + 4, 0, sizeof(int32_t), st);
-  k_tie_fix<<<gb, T, 0, st>>>(b.keys, b.vals, n, b.bounds + 4);
-  k_sort_block<<<1, kSbThreads, 0, st>>>(b.keys, b.vals, b.keys_alt, b.vals_alt, n,
-                                         b.bounds + 4);
-  launches += 2;
-  k_common_levels<<<gb, T, 0, st>>>(b.keys, n, top, nlev, b.L, b.err);
-  k_counts<<<gb, T, 0, st>>>(b.L, n, b.cnt);
-  launches += 2 + exclusive_scan(b.cnt, b.off, n, b.scan_partial, true, st);
-  k_bounds<<<1, 32, 0, st>>>(b.off, n, split, b.cap, b.bounds, b.err);
+  // node_nchild serves as the owner array of the combined tree, which counts
+  // no children
+  if (small) {
+    k_rank<<<(n + 31) / 32, 32 * kRankWarps, 0, st>>>(b.keys_alt, n, b.keys, b.vals);
+    k_front<<<1, kFrontThreads, 0, st>>>(b.keys, n, split, top, nlev, b.cap, b.L, b.off,
+                                         mode == 0 ? nullptr : b.node_nchild, b.bounds,
+                                         b.mx.lvl + kNetClimbSlot, b.err);
+    launches += 2;
+  } else {
+    // sort the high 64 bits (8 passes over 12-byte pairs), gather the full
+    // keys in that order, then order the rare ties fully;
+    // a long tie run switches on the one-block full sort (which exits otherwise)
+    launches += radix_sort(hi, b.vals, hi + n, b.vals_alt, n, b.sort_hist, b.scan_partial, st);
+    k_gather_keys<<<gb, T, 0, st>>>(b.keys_alt, b.vals, n, b.keys);
+    cudaMemsetAsync(b.bounds + 4, 0, sizeof(int32_t), st);
+    k_tie_fix<<<gb, T, 0, st>>>(b.keys, b.vals, n, b.bounds + 4);
+    k_sort_block<<<1, kSbThreads, 0, st>>>(b.keys, b.vals, b.keys_alt, b.vals_alt, n,
+                                           b.bounds + 4);
+    k_common_levels<<<gb, T, 0, st>>>(b.keys, n, top, nlev, b.L, b.err);
+    k_counts<<<gb, T, 0, st>>>(b.L, n, b.cnt);
+    launches += 5 + exclusive_scan(b.cnt, b.off, n, b.scan_partial, true, st);
+    k_bounds<<<1, 32, 0, st>>>(b.off, n, split, b.cap, b.bounds, b.err);
+    launches += 1;
+    if (mode != 0) {
+      k_owner<<<gb, T, 0, st>>>(b.off, n, b.cap, b.node_nchild);
+      launches += 1;
+    }
+  }
   // per-node passes: a grid of one thread per node for trees of up to 2n
   // nodes (the usual size), striding over the device's node count beyond
   // (the capacity can be many times the tree after a co-located start).
@@ -1239,24 +1441,27 @@ int build_trees(const BuildBuffers& b, const double* x, int n, int n_el,
                                  b.node_level, b.mx, ens, b.err);
     k_link_children<<<gcap, T, 0, st>>>(b.node_parent, b.bounds, b.cap,
                                         b.node_nchild, b.mx);
-    launches += 3;
+    launches += 2;
   } else {
-    // node_nchild serves as the owner array (the combined tree counts no children)
-    k_owner<<<gb, T, 0, st>>>(b.off, n, b.cap, b.node_nchild);
     k_topology_mixed<<<gcap, T, 0, st>>>(b.keys, b.vals, b.L, b.off, b.node_nchild, b.bounds,
                                          n, n_el, x, b.geom, b.cap, b.node_c, b.node_pt,
                                          b.node_parent, b.node_done, b.node_level, b.mx, ens);
     k_link_children<<<gcap, T, 0, st>>>(b.node_parent, b.bounds, b.cap, nullptr, b.mx);
-    launches += 4;
+    launches += 2;
   }
   if (mode == 0) {
     k_upward<<<gb, T, 0, st>>>(x, b.vals, b.L, b.off, n, split, b.geom, theta,
                                b.cap, b.bounds, b.node_c, b.node_m,
-                               b.node_skip, b.node_parent, b.node_nchild,
+                               b.mx.kids, b.node_parent, b.node_nchild,
                                b.node_done, b.node_level, b.err);
     return launches + 1;
   }
-  launches += net_moments(b, n, theta, ens, full_records, st);
+  launches += net_moments(b, n, theta, ens, full_records, small, st);
+  if (small && ens.nseg == 0) {
+    k_groups_small<<<1, 1024, 0, st>>>(b.bounds, b.cap, b.node_parent, b.node_level, b.mx,
+                                       b.mx.groups, b.mx.n_groups);
+    return launches + 1;
+  }
   // the level lists of the upward pass are free again: a single cloud keeps
   // its group-level histogram there, an ensemble has one row per cloud
   const int nsg = ens.nseg > 0 ? ens.nseg : 1;

@@ -118,8 +118,11 @@ int radix_sort(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int n,
 int build_trees(const BuildBuffers& b, const double* x, int n, int n_el,
                 double theta, int mode, cudaStream_t st, bool full_records = false);
 // The net-charge moments of the combined tree (mode 1) once its topology and
-// child tables exist.
+// child tables exist.  small: the front of a small build has zeroed
+// mx.lvl[kNetClimbSlot], and one launch takes the place of the class sort and
+// the direct sums.
+constexpr int kNetClimbSlot = 16 + 9;
 int net_moments(const BuildBuffers& b, int n, double theta, const Ensemble& ens,
-                bool full_records, cudaStream_t st);
+                bool full_records, bool small, cudaStream_t st);
 
 }  // namespace tg

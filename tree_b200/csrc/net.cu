@@ -622,14 +622,14 @@ __global__ void __launch_bounds__(kNetThreads)
 // The twigs above kMidCount: a group of 8 lanes per climb start computes its
 // twig from the children, then climbs while it is the last child to arrive
 // at the parent (fence, atomic, fence: the children's records are visible to
-// the group that completes the parent).  list[start[6] .. start[7]).
+// the group that completes the parent).  list[*begin .. *end).
 __global__ void __launch_bounds__(128)
     k_net_top(const Geom* __restrict__ geom, double theta, int cap, double4* node_c,
               const int32_t* __restrict__ node_parent, int32_t* node_done,
               const int8_t* __restrict__ node_level, MixedNodes mx, Ensemble ens,
-              const int32_t* __restrict__ start, const int32_t* __restrict__ list,
-              int32_t* err) {
-  const int b0 = start[6], b1 = start[7];
+              const int32_t* __restrict__ begin, const int32_t* __restrict__ end,
+              const int32_t* __restrict__ list, int32_t* err) {
+  const int b0 = begin ? *begin : 0, b1 = *end;
   const int lane = threadIdx.x & 31, j = lane & 7;
   const unsigned gm = 0xffu << (lane & 24);
   if (*((volatile int32_t*)err) & (kErrCapacity | kErrWalk)) return;
@@ -657,11 +657,40 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// Small builds: both kinds of direct sum and the list of climb starts in one
+// launch, straight from the nodes -- with a few thousand twigs the longest one
+// sets the time, sorted or not.  The first `gt` blocks take a thread per node,
+// the others a warp per node.  The sums are those of the two kernels above.
+__global__ void __launch_bounds__(kNetThreads)
+    k_net_small(const int32_t* __restrict__ bounds, int cap, int gt,
+                const Geom* __restrict__ geom, double theta, double4* node_c,
+                const int32_t* __restrict__ node_pt, const int8_t* __restrict__ node_level,
+                const int32_t* __restrict__ node_parent, int32_t* node_done, MixedNodes mx,
+                Ensemble ens, int32_t* climbs, int32_t* list, int full, int32_t* err) {
+  if (*((volatile int32_t*)err) & (kErrCapacity | kErrWalk)) return;
+  const int m = bounds[2] < cap ? bounds[2] : cap;
+  if (blockIdx.x < gt) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gt * blockDim.x) {
+      const int k = net_class(i, cap, node_pt, mx, node_done, true);
+      if (k == 6) list[atomicAdd(climbs, 1)] = i;
+      else if (k >= 0 && k < 5)
+        net_p2m<1>(i, 0, geom, theta, node_c, node_level, node_parent, mx, ens, full != 0);
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31, nw = ((gridDim.x - gt) * blockDim.x) >> 5;
+  for (int i = ((blockIdx.x - gt) * blockDim.x + threadIdx.x) >> 5; i < m; i += nw) {
+    if (node_pt[i] >= 0 || net_class_of(mx.count[i]) != 5) continue;  // warp-uniform
+    net_p2m<32>(i, lane, geom, theta, node_c, node_level, node_parent, mx, ens, full != 0);
+    __syncwarp();
+  }
+}
+
 // The net-charge moments of the combined tree (sort of the twigs into
 // classes, direct sums, climb) once the topology (with the leaves' positions
 // and the sorted copy xs) and the child tables exist.  Returns launches.
 int net_moments(const BuildBuffers& b, int n, double theta, const Ensemble& ens, bool full,
-                cudaStream_t st) {
+                bool small, cudaStream_t st) {
   const int T = kNetThreads;
   const int NB = (b.cap + kNetBlockNodes - 1) / kNetBlockNodes;
   int32_t* cnt = b.mx.cls;                  // 7 NB class counts
@@ -670,6 +699,17 @@ int net_moments(const BuildBuffers& b, int n, double theta, const Ensemble& ens,
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (small) {
+    int32_t* climbs = b.mx.lvl + kNetClimbSlot;
+    const int gt = (2 * n + T - 1) / T;
+    k_net_small<<<gt + sms, T, 0, st>>>(b.bounds, b.cap, gt, b.geom, theta, b.node_c, b.node_pt,
+                                        b.node_level, b.node_parent, b.node_done, b.mx, ens,
+                                        climbs, b.mx.lvl_list, full ? 1 : 0, b.err);
+    if (n <= kMidCount) return 1;  // no twig above the direct sums
+    k_net_top<<<sms, 128, 0, st>>>(b.geom, theta, b.cap, b.node_c, b.node_parent, b.node_done,
+                                   b.node_level, b.mx, ens, nullptr, climbs, b.mx.lvl_list, b.err);
+    return 2;
+  }
   const int gblk = NB < 4 * sms ? NB : 4 * sms;
   k_net_mark<<<gblk, T, 0, st>>>(b.bounds, b.cap, NB, b.node_pt, b.node_done, b.mx, cnt);
   k_net_scan<<<1, 1024, 0, st>>>(b.bounds, b.cap, NB, cnt, off, start);
@@ -686,7 +726,8 @@ int net_moments(const BuildBuffers& b, int n, double theta, const Ensemble& ens,
   k_net_p2m_warp<<<g2, T, 0, st>>>(b.geom, theta, b.node_c, b.node_level, b.node_parent,
                                    b.mx, ens, start, b.mx.lvl_list, full ? 1 : 0, b.err);
   k_net_top<<<sms, 128, 0, st>>>(b.geom, theta, b.cap, b.node_c, b.node_parent, b.node_done,
-                                 b.node_level, b.mx, ens, start, b.mx.lvl_list, b.err);
+                                 b.node_level, b.mx, ens, start + 6, start + 7, b.mx.lvl_list,
+                                 b.err);
   return 6;
 }
 
