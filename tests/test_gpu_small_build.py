@@ -1,6 +1,6 @@
-"""The small build (counting sort, one-block passes) at its edges: trees equal
-to the oracle's bit for bit on the FP64 path, and on the mixed path the sorted
-particles, cells and moments of every twig."""
+"""The small build (counting sort, one-block passes) and the sort without scans at
+their edges: trees equal to the oracle's bit for bit on the FP64 path, and on the
+mixed path the sorted particles, cells and moments of every twig."""
 import numpy as np
 import pytest
 
@@ -23,7 +23,7 @@ def _points(n, seed, tight):
 
 @pytest.mark.parametrize("tight", [False, True])
 @pytest.mark.parametrize("n_el,n_ion", [(1, 0), (1, 2), (40, 0), (0, 33), (700, 333), (2100, 2300),
-                                        (8191, 8193), (8192, 8193)])
+                                        (6143, 6145), (6144, 6145), (8192, 8193)])
 def test_fp64_trees(device_lib, oracle_lib, n_el, n_ion, tight):
     x_el, x_ion = _points(n_el, n_el + 1, tight), _points(n_ion, n_ion + 2, tight)
     with api.TreeForce(n_el, n_ion, api.Config(theta=0.7, precision=api.PREC_FP64)) as tf:
@@ -44,8 +44,8 @@ def test_fp64_trees(device_lib, oracle_lib, n_el, n_ion, tight):
 
 
 @pytest.mark.parametrize("tight", [False, True])
-@pytest.mark.parametrize("n_el,n_ion", [(1, 1), (40, 33), (1024, 1024), (1024, 1025), (8192, 8192),
-                                        (8192, 8193)])
+@pytest.mark.parametrize("n_el,n_ion", [(1, 1), (40, 33), (1024, 1024), (1024, 1025), (6144, 6144),
+                                        (6144, 6145), (131072, 131072), (131073, 131072)])
 def test_mixed_tree(device_lib, n_el, n_ion, tight):
     x_el, x_ion = _points(n_el, n_el + 1, tight), _points(n_ion, n_ion + 2, tight)
     cfg = api.Config(theta=0.7, physics=api.PHYS_KELBG, precision=api.PREC_MIXED)

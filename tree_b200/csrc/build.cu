@@ -373,11 +373,20 @@ constexpr int kRsIters = 8;                        // items per lane
 constexpr int kRsTile = kRsThreads * kRsIters;     // 2048 items per block
 constexpr int kRsBins = 256;
 
+// Up to this many blocks (262,144 keys) a scatter block adds up the counts of
+// the blocks before it by itself, from rows [nb][256]: at most 128 loads a
+// thread, against three launches of a scan a pass.  Build us in the step graph,
+// mixed | FP64 path: N = 16,400 314 -> 254 | 239 -> 190, N = 65,536 341 -> 282 |
+// 265 -> 211, N = 262,144 457 -> 423 | 417 -> 375 (with k_common_levels and
+// k_owner taking in two more launches).  The rows that all blocks read grow
+// with the square of their number.
+constexpr int kRsRowBlocks = 128;
+
 int radix_blocks(int n) { return (n + kRsTile - 1) / kRsTile; }
 
-template <class K>
+template <class K, bool ROWS>
 __global__ void k_rs_hist(const K* __restrict__ keys, int n, int shift,
-                          int32_t* hist /* [256][nb] */) {
+                          int32_t* hist /* [256][nb]; ROWS: [nb][256] */) {
   __shared__ int32_t h[kRsBins];
   for (int b = threadIdx.x; b < kRsBins; b += blockDim.x) h[b] = 0;
   __syncthreads();
@@ -388,26 +397,42 @@ __global__ void k_rs_hist(const K* __restrict__ keys, int n, int shift,
   }
   __syncthreads();
   for (int b = threadIdx.x; b < kRsBins; b += blockDim.x)
-    hist[(int64_t)b * gridDim.x + blockIdx.x] = h[b];
+    hist[ROWS ? blockIdx.x * kRsBins + b : (int64_t)b * gridDim.x + blockIdx.x] = h[b];
 }
 
 // Stable scatter: tile order is warp-major (warp w owns items
 // [w*32*kRsIters, (w+1)*32*kRsIters) of the tile), then iteration, then lane.
-template <class K>
+template <class K, bool ROWS>
 __global__ void __launch_bounds__(kRsThreads)
     k_rs_scatter(const K* __restrict__ keys_in,
                  const uint32_t* __restrict__ vals_in, int n, int shift,
-                 const int32_t* __restrict__ offs /* scanned [256][nb] */,
+                 const int32_t* __restrict__ offs /* scanned [256][nb]; ROWS: counts [nb][256] */,
                  K* __restrict__ keys_out,
                  uint32_t* __restrict__ vals_out) {
   __shared__ int32_t whist[kRsWarps][kRsBins];
   __shared__ int32_t base_s[kRsBins];
   int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int b = threadIdx.x; b < kRsBins; b += blockDim.x) {
-    base_s[b] = offs[(int64_t)b * gridDim.x + blockIdx.x];
+  static_assert(kRsThreads == kRsBins && kRsThreads == kScanThreads, "a thread per digit");
+  if (ROWS) {
+    const int d = threadIdx.x, nb = gridDim.x;
+    int32_t before = 0, all = 0;
+    for (int b0 = 0; b0 < nb; b0 += 16) {
+      int32_t v[16];
 #pragma unroll
-    for (int ww = 0; ww < kRsWarps; ++ww) whist[ww][b] = 0;
+      for (int j = 0; j < 16; ++j) v[j] = b0 + j < nb ? offs[(b0 + j) * kRsBins + d] : 0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        all += v[j];
+        if (b0 + j < (int)blockIdx.x) before += v[j];
+      }
+    }
+    __shared__ int32_t tot;
+    base_s[d] = block_excl_scan(all, &tot) + before;
+  } else {
+    base_s[threadIdx.x] = offs[(int64_t)threadIdx.x * gridDim.x + blockIdx.x];
   }
+#pragma unroll
+  for (int ww = 0; ww < kRsWarps; ++ww) whist[ww][threadIdx.x] = 0;
   __syncthreads();
   int64_t wbase = (int64_t)blockIdx.x * kRsTile + (int64_t)w * (32 * kRsIters);
   K k[kRsIters];
@@ -465,10 +490,15 @@ int radix_sort(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int n,
   uint32_t* vout = vals_alt;
   for (int pass = first_byte; pass < (int)sizeof(K); ++pass) {
     int shift = pass * 8;
-    k_rs_hist<K><<<nb, kRsThreads, 0, st>>>(kin, n, shift, hist);
-    launches += 2 + exclusive_scan(hist, hist, kRsBins * nb, partial, false, st);
-    k_rs_scatter<K><<<nb, kRsThreads, 0, st>>>(kin, vin, n, shift, hist, kout,
-                                               vout);
+    launches += 2;
+    if (nb <= kRsRowBlocks) {
+      k_rs_hist<K, true><<<nb, kRsThreads, 0, st>>>(kin, n, shift, hist);
+      k_rs_scatter<K, true><<<nb, kRsThreads, 0, st>>>(kin, vin, n, shift, hist, kout, vout);
+    } else {
+      k_rs_hist<K, false><<<nb, kRsThreads, 0, st>>>(kin, n, shift, hist);
+      launches += exclusive_scan(hist, hist, kRsBins * nb, partial, false, st);
+      k_rs_scatter<K, false><<<nb, kRsThreads, 0, st>>>(kin, vin, n, shift, hist, kout, vout);
+    }
     K* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;
   }
@@ -629,18 +659,16 @@ __device__ __forceinline__ int8_t common_level(key128 a, key128 b, int top, int 
   return (int8_t)(lev < nlev ? lev : nlev);
 }
 
-__global__ void k_common_levels(const key128* __restrict__ keys, int n,
-                                int top, int nlev, int8_t* L, int32_t* err) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
+// ... and the nodes that each particle emits.
+__global__ void k_common_levels(const key128* __restrict__ keys, int n, int top, int nlev,
+                                int8_t* L, int32_t* cnt, int32_t* err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  L[p] = p + 1 < n ? common_level(keys[p], keys[p + 1], top, nlev, err) : (int8_t)-1;
-}
-
-__global__ void k_counts(const int8_t* __restrict__ L, int n, int32_t* cnt) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  int lo, hi;
-  lo_hi(L, p, lo, hi);
+  const key128 k = keys[p];
+  const int lo = p > 0 ? common_level(keys[p - 1], k, top, nlev, err) : -1;
+  int hi = p + 1 < n ? common_level(k, keys[p + 1], top, nlev, err) : -1;
+  L[p] = (int8_t)hi;
+  if (lo < 0 && hi < 0) hi = 0;  // as lo_hi
   cnt[p] = (hi > lo ? hi - lo : 0) + 1;
 }
 
@@ -818,6 +846,16 @@ __global__ void k_topology(const key128* __restrict__ keys,
                               : twig_index_before(keys, L, off, sb, p, depth - 1, top);
 }
 
+// me, m: nodes of the first tree, of both.
+__device__ __forceinline__ void write_bounds(int me, int m, int cap, int32_t* bounds,
+                                             int32_t* err) {
+  if (m > cap) set_error(err, kErrCapacity);
+  bounds[0] = 0;
+  bounds[1] = me < cap ? me : cap;
+  bounds[2] = m < cap ? m : cap;
+  bounds[3] = m;  // untruncated node count (for capacity growth)
+}
+
 // ------------------------------------------- combined-tree topology ----
 // The combined tree of the mixed path is written one thread per node rather
 // than one per particle: no lane waits on another's emission loop.  Node i
@@ -829,8 +867,10 @@ __global__ void k_topology(const key128* __restrict__ keys,
 // write their position (w = -1, the walk's leaf mark) and the sorted copy
 // xs (w = 1 for ions).  The child table is cleared here and filled by
 // k_link_children; per-node skip and child counts are not needed.
-__global__ void k_owner(const int32_t* __restrict__ off, int n, int cap, int32_t* owner) {
+__global__ void k_owner(const int32_t* __restrict__ off, int n, int cap, int32_t* owner,
+                        int32_t* bounds, int32_t* err) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p == 0) write_bounds(off[n], off[n], cap, bounds, err);  // one tree: k_bounds
   if (p >= n) return;
   const int e = off[p + 1] < cap ? off[p + 1] : cap;
   for (int i = off[p]; i < e; ++i) owner[i] = p;
@@ -948,33 +988,24 @@ __global__ void k_roots(const int32_t* __restrict__ off,
   if (c < nseg) roots[c] = off[start[c]];
 }
 
-// me, m: nodes of the first tree, of both.
-__device__ __forceinline__ void write_bounds(int me, int m, int cap, int32_t* bounds,
-                                             int32_t* err) {
-  if (m > cap) set_error(err, kErrCapacity);
-  bounds[0] = 0;
-  bounds[1] = me < cap ? me : cap;
-  bounds[2] = m < cap ? m : cap;
-  bounds[3] = m;  // untruncated node count (for capacity growth)
-}
-
 __global__ void k_bounds(const int32_t* __restrict__ off, int n, int n_el,
                          int cap, int32_t* bounds, int32_t* err) {
   if (threadIdx.x == 0) write_bounds(off[n_el], off[n], cap, bounds, err);
 }
 
 // ------------------------------------------------ front of a small build ----
-// Up to kFrontMax particles two launches do what takes 50 above (the radix
-// sort's 40 among them): a small build is a chain of launches, 2.5 to 4 us each
+// Up to kFrontMax particles two launches do what takes 24 to 50 above (the radix
+// sort's 16 or 40 among them): a small build is a chain of launches, 2.5 to 4 us each
 // in a step graph, on arrays that hardly fill one SM.  With k_bbox_small,
 // k_net_small and k_groups_small a build takes (us in the step graph, mixed |
 // FP64 path):
 //   N = 1,000   194 -> 56  | 199 -> 70
 //   N = 4,000   254 -> 96  | 237 -> 92
 //   N = 8,192   271 -> 147 | 257 -> 130
-//   N = 16,384  317 -> 303 | 273 -> 248, where the n^2 comparisons catch up.
+// The comparisons grow with n^2: at 16,384 it is 302 us against 254 for the
+// passes of k_rs_hist and k_rs_scatter, at 12,288 about 211 against 245.
 constexpr int kFrontThreads = 1024;
-constexpr int kFrontItems = 16;
+constexpr int kFrontItems = 12;
 constexpr int kFrontMax = kFrontThreads * kFrontItems;
 
 // Sorts by counting: the rank of a key is the number of keys below it (equal
@@ -1023,7 +1054,7 @@ __global__ void __launch_bounds__(32 * kRankWarps)
   }
 }
 
-// What follows the sort, in one block: k_common_levels, k_counts, the scan,
+// What follows the sort, in one block: k_common_levels, the scan,
 // k_bounds, (owner != nullptr) k_owner, and the zero of *climbs (k_net_small's
 // list of climb starts).
 struct FrontSmem {
@@ -1415,15 +1446,10 @@ int build_trees(const BuildBuffers& b, const double* x, int n, int n_el,
     k_tie_fix<<<gb, T, 0, st>>>(b.keys, b.vals, n, b.bounds + 4);
     k_sort_block<<<1, kSbThreads, 0, st>>>(b.keys, b.vals, b.keys_alt, b.vals_alt, n,
                                            b.bounds + 4);
-    k_common_levels<<<gb, T, 0, st>>>(b.keys, n, top, nlev, b.L, b.err);
-    k_counts<<<gb, T, 0, st>>>(b.L, n, b.cnt);
+    k_common_levels<<<gb, T, 0, st>>>(b.keys, n, top, nlev, b.L, b.cnt, b.err);
     launches += 5 + exclusive_scan(b.cnt, b.off, n, b.scan_partial, true, st);
-    k_bounds<<<1, 32, 0, st>>>(b.off, n, split, b.cap, b.bounds, b.err);
-    launches += 1;
-    if (mode != 0) {
-      k_owner<<<gb, T, 0, st>>>(b.off, n, b.cap, b.node_nchild);
-      launches += 1;
-    }
+    if (mode == 0) k_bounds<<<1, 32, 0, st>>>(b.off, n, split, b.cap, b.bounds, b.err);
+    else k_owner<<<gb, T, 0, st>>>(b.off, n, b.cap, b.node_nchild, b.bounds, b.err);
   }
   // per-node passes: a grid of one thread per node for trees of up to 2n
   // nodes (the usual size), striding over the device's node count beyond
