@@ -51,6 +51,28 @@ struct StepGraph {
   int64_t replays = 0;   // replays during the current call
 };
 
+// The small device results of a call, one block on the device and its pinned
+// copy: a call ends with one read-back and one synchronisation.  A force call of
+// 4,096 particles took 0.474 ms (mixed) and 0.617 ms (FP64) when each result was
+// its own pageable copy; with this block and the staging below 0.346 and 0.505 ms.
+struct Status {
+  int32_t err;        // BuildBuffers::err
+  int32_t bounds[5];  // BuildBuffers::bounds
+  int32_t series_count;
+  int32_t pad;
+  // [0..3] this step's walk counts, [4..7] running totals of the handle,
+  // [8] this step's cells in local expansions, [9] their running total
+  unsigned long long counters[16];
+  double diag[8];     // [0..3] epot, [4..7] kinetic sums
+};
+
+// Particles up to which tree_gpu_force moves positions and forces through the
+// handle's pinned block: below, a pageable copy is mostly its own overhead (a
+// fixed cost per copy and per wait).  Above, a host copy in between costs as much
+// as it saves: at N = 1M a call is 1.8 ms longer than its device work, and moving
+// the arrays through pinned slots with four threads took only 0.5 ms off that.
+constexpr int64_t kStageParticles = 16384;
+
 }  // namespace
 
 struct tree_gpu_handle {
@@ -80,10 +102,13 @@ struct tree_gpu_handle {
   int32_t* smp_count = nullptr;
   int64_t smp_cap = 0;
   uint32_t* rdf = nullptr;
-  unsigned long long* counters = nullptr;
+  Status* status = nullptr;               // device
+  unsigned long long* counters = nullptr;  // in status
   double* partial = nullptr;
-  double* diag = nullptr;  // [0..3] epot, [4..7] kinetic sums
-  int32_t* h_pinned = nullptr;  // small pinned readback area
+  double* diag = nullptr;                  // in status
+  Status* h_pinned = nullptr;              // pinned: status, RDF bins, staging
+  unsigned long long* h_rdf = nullptr;     // 2 x kRdfBins
+  double* h_stage = nullptr;               // 3 n doubles up to kStageParticles, else null
   bool has_state = false;
   double lam[3] = {1, 1, 1};
   tree_gpu_timing timing{};
@@ -203,18 +228,16 @@ int alloc_all(tree_gpu_handle* h) {
   if ((rc = dalloc(h, &b.scan_partial, (size_t)sp + 1))) return rc;
   if ((rc = dalloc(h, &b.bbox, 12))) return rc;
   if ((rc = dalloc(h, &b.geom, 2))) return rc;
-  if ((rc = dalloc(h, &b.bounds, 5))) return rc;
-  if ((rc = dalloc(h, &b.err, 1))) return rc;
+  if ((rc = dalloc(h, &h->status, 1))) return rc;
+  b.bounds = h->status->bounds;  // addresses in device memory, not read here
+  b.err = &h->status->err;
+  h->series_count = &h->status->series_count;
+  h->counters = h->status->counters;
+  h->diag = h->status->diag;
   if ((rc = dalloc(h, &h->rdf, 2 * (size_t)tg::kRdfBins))) return rc;
-  if ((rc = dalloc(h, &h->counters, 16))) return rc;
-  // [0..3] this step's walk counts, [4..7] running totals of the handle,
-  // [8] this step's cells in local expansions, [9] their running total
-  if (cudaMemset(h->counters, 0, 16 * sizeof(unsigned long long)) != cudaSuccess)
-    return fail(h, TREE_GPU_ERR_CUDA, "counter initialisation failed");
+  CK(cudaMemsetAsync(h->status, 0, sizeof(Status), h->st));
   if ((rc = dalloc(h, &h->partial, 4 * (size_t)tg::kdk_partials_needed(n) + 4)))
     return rc;
-  if ((rc = dalloc(h, &h->diag, 8))) return rc;
-  CK(cudaMemsetAsync(h->diag, 0, 8 * sizeof(double), h->st));
   if (tg::mixed_alloc_particles(h->mb, n))
     return fail(h, TREE_GPU_ERR_CUDA, "mixed particle alloc");
   h->b.mx = tg::mixed_nodes(h->mb);
@@ -226,12 +249,12 @@ void free_all(tree_gpu_handle* h) {
   tg::BuildBuffers& b = h->b;
   void* ptrs[] = {h->x, h->v, h->f, h->epot_part, b.keys, b.keys_alt, b.vals,
                   b.vals_alt, b.L, b.cnt, b.off, b.sort_hist, b.scan_partial,
-                  b.bbox, b.geom, b.bounds, b.err, b.node_c, b.node_m,
+                  b.bbox, b.geom, h->status, b.node_c, b.node_m,
                   b.node_skip, b.node_pt, b.node_parent, b.node_nchild,
-                  b.node_done, b.node_level, h->rdf, h->counters, h->partial,
-                  h->diag, h->mlp_params, h->mlp_stats, h->mlp_packed,
+                  b.node_done, b.node_level, h->rdf, h->partial, h->mlp_params,
+                  h->mlp_stats, h->mlp_packed,
                   h->smp_feats, h->smp_labels, h->smp_extra, h->smp_count,
-                  h->series, h->series_count, h->rdf64, h->ens_start,
+                  h->series, h->rdf64, h->ens_start,
                   h->ens_elec_end, h->ens_roots, h->ens_glvl, h->cloud_pk,
                   h->ion_flag, h->cloud_sums, h->direct_ws};
   for (void* p : ptrs)
@@ -322,16 +345,14 @@ void enqueue_force(tree_gpu_handle* h, bool with_rdf, EventSet* ev) {
   tg::epot_sum(h->epot_part, h->n, h->partial, h->diag, h->counters, st);
 }
 
-// Reads the error word and node counts after a synchronised call.
+// Ends a call's device work: reads the status block back, waits for the
+// stream, and turns the error word into a return code.
 int check_device_status(tree_gpu_handle* h, bool* grow) {
   *grow = false;
-  int32_t* hp = h->h_pinned;
-  CK(cudaMemcpyAsync(hp, h->b.err, sizeof(int32_t), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(hp + 1, h->b.bounds, 4 * sizeof(int32_t),
-                     cudaMemcpyDeviceToHost, h->st));
+  CK(cudaMemcpyAsync(h->h_pinned, h->status, sizeof(Status), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
-  int32_t err = hp[0];
-  h->timing.n_nodes = hp[1 + 3];
+  const int32_t err = h->h_pinned->err;
+  h->timing.n_nodes = h->h_pinned->bounds[3];
   if (err & tg::kErrNonFinite)
     return fail(h, TREE_GPU_ERR_NONFINITE, "non-finite particle position");
   if (err & tg::kErrDepth)
@@ -346,7 +367,7 @@ int check_device_status(tree_gpu_handle* h, bool* grow) {
 }
 
 int grow_nodes(tree_gpu_handle* h) {
-  int need = h->h_pinned[1 + 3];
+  int need = h->h_pinned->bounds[3];
   if (need <= h->b.cap) need = h->b.cap;
   int64_t cap = (int64_t)need + need / 4 + 64;
   if (cap > 0x7fffffff) return fail(h, TREE_GPU_ERR_CAPACITY, "node count overflow");
@@ -354,9 +375,9 @@ int grow_nodes(tree_gpu_handle* h) {
   return alloc_nodes(h, (int)cap);
 }
 
+// The counts that the last check_device_status read back.
 void read_counters(tree_gpu_handle* h) {
-  unsigned long long c[16] = {};
-  cudaMemcpy(c, h->counters, sizeof(c), cudaMemcpyDeviceToHost);
+  const unsigned long long* c = h->h_pinned->counters;
   h->timing.n_m2p = (int64_t)c[0];
   h->timing.n_p2p = (int64_t)c[1];
   h->timing.n_mac_net = (int64_t)c[2];
@@ -378,12 +399,21 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
 }
 
 // Computes forces of the current device positions, growing the node arrays
-// when the tree did not fit.
-int force_device(tree_gpu_handle* h, bool with_rdf) {
+// when the tree did not fit.  With `stage`, the forces and RDF bins also go to
+// the pinned block before the wait.
+int force_device(tree_gpu_handle* h, bool with_rdf, bool stage = false) {
   for (int attempt = 0; attempt < 3; ++attempt) {
     EventSet& ev = events_for(h, 0);
     enqueue_force(h, with_rdf, &ev);
     CK(cudaGetLastError());
+    if (stage) {
+      if (h->h_stage && h->n > 0)
+        CK(cudaMemcpyAsync(h->h_stage, h->f, 3 * sizeof(double) * (size_t)h->n,
+                           cudaMemcpyDeviceToHost, h->st));
+      if (with_rdf)
+        CK(cudaMemcpyAsync(h->h_rdf, h->rdf, 2 * sizeof(uint32_t) * tg::kRdfBins,
+                           cudaMemcpyDeviceToHost, h->st));
+    }
     bool grow = false;
     int rc = check_device_status(h, &grow);
     if (rc) return rc;
@@ -498,8 +528,9 @@ void free_graphs(tree_gpu_handle* h) {
 // always on the last step when sample_last; samples go to the series buffer
 // when it is set.  With rdf, the near-field pair counts of every step are
 // added to h->rdf64.
+// The first `records` sample records go to `series` (pageable host memory).
 int run_impl(tree_gpu_handle* h, double dt, int32_t nsteps, int32_t nsamp,
-             bool sample_last, bool rdf) {
+             bool sample_last, bool rdf, double* series = nullptr, int64_t records = 0) {
   const int n = h->n, ne = (int)h->n_el;
   const tree_gpu_params& p = h->prm;
   events_for(h, (size_t)nsteps + 1);  // grow first: references below stay valid
@@ -536,6 +567,12 @@ int run_impl(tree_gpu_handle* h, double dt, int32_t nsteps, int32_t nsamp,
   }
   cudaEventRecord(et.e[1], h->st);
   CK(cudaGetLastError());
+  if (rdf)
+    CK(cudaMemcpyAsync(h->h_rdf, h->rdf64, 2 * sizeof(unsigned long long) * tg::kRdfBins,
+                       cudaMemcpyDeviceToHost, h->st));
+  if (records > 0)
+    CK(cudaMemcpyAsync(series, h->series, 6 * sizeof(double) * (size_t)records,
+                       cudaMemcpyDeviceToHost, h->st));
   bool grow = false;
   int rc = check_device_status(h, &grow);
   if (rc) return rc;
@@ -628,10 +665,16 @@ int tree_gpu_create(const tree_gpu_params* params, int64_t n_el, int64_t n_ion,
       break;
     }
     h->st = h->own_st;
-    if (cudaMallocHost((void**)&h->h_pinned, 64) != cudaSuccess) {
+    const size_t rdf_bytes = 2 * sizeof(unsigned long long) * tg::kRdfBins;
+    const bool stage = h->n > 0 && h->n <= kStageParticles;
+    if (cudaMallocHost((void**)&h->h_pinned, sizeof(Status) + rdf_bytes +
+                                                 (stage ? 3 * sizeof(double) * h->n : 0)) !=
+        cudaSuccess) {
       rc = fail(h, TREE_GPU_ERR_CUDA, "pinned alloc failed");
       break;
     }
+    h->h_rdf = reinterpret_cast<unsigned long long*>(h->h_pinned + 1);
+    if (stage) h->h_stage = reinterpret_cast<double*>(h->h_rdf + 2 * tg::kRdfBins);
     rc = alloc_all(h);
   } while (0);
   if (rc != TREE_GPU_OK) {
@@ -675,9 +718,16 @@ int tree_gpu_force(tree_gpu_handle* h, const double* x_el, const double* x_ion,
     return fail(h, TREE_GPU_ERR_ARG, "null particle buffer");
   const size_t be = 3 * sizeof(double) * (size_t)h->n_el;
   const size_t bi = 3 * sizeof(double) * (size_t)h->n_ion;
-  if (be) CK(cudaMemcpyAsync(h->x, x_el, be, cudaMemcpyHostToDevice, h->st));
-  if (bi)
-    CK(cudaMemcpyAsync(h->x + 3 * h->n_el, x_ion, bi, cudaMemcpyHostToDevice, h->st));
+  double* stage = h->h_stage;
+  if (stage) {
+    if (be) std::memcpy(stage, x_el, be);
+    if (bi) std::memcpy(stage + 3 * h->n_el, x_ion, bi);
+    CK(cudaMemcpyAsync(h->x, stage, be + bi, cudaMemcpyHostToDevice, h->st));
+  } else {
+    if (be) CK(cudaMemcpyAsync(h->x, x_el, be, cudaMemcpyHostToDevice, h->st));
+    if (bi)
+      CK(cudaMemcpyAsync(h->x + 3 * h->n_el, x_ion, bi, cudaMemcpyHostToDevice, h->st));
+  }
   bool with_rdf = rdf_ei || rdf_ii;
   int rc;
   if (h->prm.mac == TREE_GPU_MAC_LEARNED && h->prm.precision == TREE_GPU_PREC_MIXED) {
@@ -687,25 +737,23 @@ int tree_gpu_force(tree_gpu_handle* h, const double* x_el, const double* x_ion,
     if ((rc = force_device(h, false))) return rc;
     h->has_fprev = true;
   }
-  rc = force_device(h, with_rdf);
+  rc = force_device(h, with_rdf, true);
   h->has_fprev = false;
   h->has_state = false;  // the device positions are now this call's, not a state
   if (rc) return rc;
-  if (be) CK(cudaMemcpyAsync(f_el, h->f, be, cudaMemcpyDeviceToHost, h->st));
-  if (bi)
-    CK(cudaMemcpyAsync(f_ion, h->f + 3 * h->n_el, bi, cudaMemcpyDeviceToHost, h->st));
-  double ep[4];
-  CK(cudaMemcpyAsync(ep, h->diag, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-  std::vector<uint32_t> hr;
-  if (with_rdf) {
-    hr.resize(2 * (size_t)tg::kRdfBins);
-    CK(cudaMemcpyAsync(hr.data(), h->rdf, hr.size() * sizeof(uint32_t),
-                       cudaMemcpyDeviceToHost, h->st));
+  if (stage) {
+    if (be) std::memcpy(f_el, stage, be);
+    if (bi) std::memcpy(f_ion, stage + 3 * h->n_el, bi);
+  } else {
+    if (be) CK(cudaMemcpyAsync(f_el, h->f, be, cudaMemcpyDeviceToHost, h->st));
+    if (bi)
+      CK(cudaMemcpyAsync(f_ion, h->f + 3 * h->n_el, bi, cudaMemcpyDeviceToHost, h->st));
+    CK(cudaStreamSynchronize(h->st));
   }
-  CK(cudaStreamSynchronize(h->st));
-  if (epot_e) *epot_e = ep[0];
-  if (epot_i) *epot_i = ep[1];
+  if (epot_e) *epot_e = h->h_pinned->diag[0];
+  if (epot_i) *epot_i = h->h_pinned->diag[1];
   if (with_rdf) {
+    const uint32_t* hr = reinterpret_cast<const uint32_t*>(h->h_rdf);
     for (int i = 0; i < tg::kRdfBins; ++i) {
       if (rdf_ei) rdf_ei[i] += hr[i];
       if (rdf_ii) rdf_ii[i] += hr[tg::kRdfBins + i];
@@ -782,8 +830,7 @@ int tree_gpu_step(tree_gpu_handle* h, double dt, int32_t nsteps,
   h->series = keep;
   if (rc) return rc;
   if (out) {
-    double d[8];
-    CK(cudaMemcpy(d, h->diag, sizeof(d), cudaMemcpyDeviceToHost));
+    const double* d = h->h_pinned->diag;
     out->epot_e = d[0];
     out->epot_i = d[1];
     out->mv2_el = d[4];
@@ -814,7 +861,6 @@ int tree_gpu_run(tree_gpu_handle* h, double dt, int32_t nsteps, int32_t nsamp,
   if (want_series && nsamples > h->series_cap) {
     const int cap = (int)std::min<int64_t>(nsamples + 16, 1 << 24);
     if (dalloc(h, &h->series, 6 * (size_t)cap)) return TREE_GPU_ERR_CUDA;
-    if (!h->series_count && dalloc(h, &h->series_count, 1)) return TREE_GPU_ERR_CUDA;
     h->series_cap = cap;
     ++h->epoch;
   }
@@ -823,19 +869,18 @@ int tree_gpu_run(tree_gpu_handle* h, double dt, int32_t nsteps, int32_t nsamp,
     ++h->epoch;
   }
   if (rdf) CK(cudaMemsetAsync(h->rdf64, 0, 2 * sizeof(unsigned long long) * tg::kRdfBins, h->st));
-  if (h->series_count) CK(cudaMemsetAsync(h->series_count, 0, sizeof(int32_t), h->st));
+  CK(cudaMemsetAsync(h->series_count, 0, sizeof(int32_t), h->st));
   double* keep = h->series;
   if (!want_series) h->series = nullptr;  // sample steps still refresh the sums
   const int64_t nloop0 = h->nloop;
-  int rc = run_impl(h, dt, nsteps, nsamp, false, rdf);
+  const int64_t want =
+      want_series ? std::min<int64_t>(nsamples, std::min(series_cap, h->series_cap)) : 0;
+  std::vector<double> buf(6 * (size_t)want);
+  int rc = run_impl(h, dt, nsteps, nsamp, false, rdf, buf.data(), want);
   h->series = keep;
   if (rc) return rc;
   if (want_series) {
-    int32_t cnt = 0;
-    CK(cudaMemcpy(&cnt, h->series_count, sizeof(int32_t), cudaMemcpyDeviceToHost));
-    const int32_t m = std::min<int32_t>(cnt, series_cap);
-    std::vector<double> buf(6 * (size_t)std::max<int32_t>(m, 1));
-    if (m) CK(cudaMemcpy(buf.data(), h->series, 6 * sizeof(double) * m, cudaMemcpyDeviceToHost));
+    const int32_t m = (int32_t)std::min<int64_t>(h->h_pinned->series_count, want);
     int64_t nl = (nloop0 / nsamp + 1) * nsamp;  // first sample step of the call
     for (int32_t k = 0; k < m; ++k, nl += nsamp) {
       series[k].nloop = nl;
@@ -849,9 +894,7 @@ int tree_gpu_run(tree_gpu_handle* h, double dt, int32_t nsteps, int32_t nsamp,
     if (n_series) *n_series = m;
   }
   if (rdf) {
-    std::vector<unsigned long long> hr(2 * (size_t)tg::kRdfBins);
-    CK(cudaMemcpy(hr.data(), h->rdf64, hr.size() * sizeof(unsigned long long),
-                  cudaMemcpyDeviceToHost));
+    const unsigned long long* hr = h->h_rdf;
     for (int i = 0; i < tg::kRdfBins; ++i) {
       if (rdf_ei) rdf_ei[i] += (int64_t)hr[i];
       if (rdf_ii) rdf_ii[i] += (int64_t)hr[tg::kRdfBins + i];
