@@ -18,14 +18,17 @@
 
 namespace tg {
 
-// What bounds it: FP64 issue and the latency of dependent FP64 operations at
-// 16 warps per SM (128 registers, 12 KB of shared memory a warp); the memory
-// side is served by L1 and L2.  At N = 262,144 (theta 0.5, reference laws,
-// RDF) the walk takes 25.2 ms, of which the FP64 pipe is busy about half; one
-// thread per target with 20 IEEE divisions per cell took 58.9 ms, at 16.5 of
-// 32 lanes active, and at N = 4,096, where it left one warp per SM, 7.3 ms
-// against 0.31 ms.  12 warps (156 registers) and 20 warps (96 registers,
-// spills) per SM were slower: 27.7 and 30.6 ms.
+// What bounds it: instruction issue and the latency of dependent operations at
+// 16 warps per SM (128 registers, 12 KB of shared memory a warp); the FP64 pipe
+// is busy less than half of the time, the memory side is served by L1 and L2.
+// At N = 262,144 (theta 0.5, reference laws, RDF) the walk takes 23.4 ms, half of
+// it walking and summing, half evaluating: 58.9 ms with one thread per target
+// and 20 IEEE divisions per cell (16.5 of 32 lanes active), 25.2 with quotients
+// of three operations.  At N = 4,096 it takes 0.30 ms against 7.3,
+// where a thread per target left one warp per SM.  Per SM, 12 warps (156
+// registers) and 20 (96, spills) were slower, 27.7 and 30.6 ms when 16 took 25.2;
+// so were blocks of one warp (26.2), a stack of 768 entries (26.2: fewer nodes at
+// a time near its limit).
 constexpr int kW64Warps = 4;
 constexpr int kW64Threads = 32 * kW64Warps;
 constexpr int kW64Blocks = 4;    // per SM
@@ -69,39 +72,57 @@ __device__ __forceinline__ bool mac64(double w, double r2) {
   return w < sqrt(r2);
 }
 
-// a / b from y = RN(1/b): one Newton correction of a y with an exact residual
-// rounds to the IEEE quotient (Markstein, "Computation of elementary functions
-// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const double q = a * y;
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
+// Division by b with a reciprocal of twice the working precision, hi + lo =
+// 1/b (1 + d) with |d| < 2^-101: a hi + a lo, rounded once, is the IEEE quotient
+// unless that lies within 2^-47 ulp of the middle between two numbers (an ulp
+// off in one quotient of 10^14).  The correction of an estimate y by its exact
+// residual e = 1 - b y and the series of 1 / (1 - e) are the long division of
+// Karp and Markstein ("High-precision division and square root", ACM Trans.
+// Math. Softw. 23(4), 1997).  A quotient is two operations, against three with
+// a residual of its own (and about 12 for an IEEE division).
+struct Divisor {
+  double hi, lo;
+  // y within 2^-47 of 1/b, relatively
+  __device__ __forceinline__ Divisor(double b, double y) : hi(y) {
+    const double e = __fma_rn(-b, y, 1.0);
+    lo = __fma_rn(e, e, e) * y;
+  }
+  __device__ __forceinline__ double inv() const { return hi + lo; }
+  __device__ __forceinline__ double operator()(double a) const {
+    return __fma_rn(a, hi, a * lo);
+  }
+};
+
+// sqrt(r2) from y = rsqrt(r2), by the same correction.
+__device__ __forceinline__ double sqrt_by(double r2, double y) {
+  const double g = r2 * y;
+  return __fma_rn(__fma_rn(-g, g, r2), 0.5 * y, g);
 }
 
-// The far field's divisors r, r^3, r^5, r^7: 28 quotients share 4 reciprocals.
+// The far field's divisors r, r^3, r^5, r^7: one rsqrt serves the root and the
+// reciprocals of 28 quotients.
 struct SharedDivisors {
-  double b1, b3, b5, b7, y1, y3, y5, y7;
-  __device__ __forceinline__ SharedDivisors(double r2, double r_) {
-    b1 = r_;
-    b3 = r2 * r_;
-    b5 = b3 * r2;
-    b7 = b5 * r2;
-    y1 = __drcp_rn(b1);
-    y3 = __drcp_rn(b3);
-    y5 = __drcp_rn(b5);
-    y7 = __drcp_rn(b7);
-  }
-  __device__ __forceinline__ double inv_R3() const { return y3; }
-  __device__ __forceinline__ double r(double a) const { return div_by(a, b1, y1); }
-  __device__ __forceinline__ double R3(double a) const { return div_by(a, b3, y3); }
-  __device__ __forceinline__ double R5(double a) const { return div_by(a, b5, y5); }
-  __device__ __forceinline__ double R7(double a) const { return div_by(a, b7, y7); }
+  Divisor d1, d3, d5, d7;
+  __device__ __forceinline__ SharedDivisors(double r2, double r_, double y, double y2,
+                                            double y3, double y5)
+      : d1(r_, y), d3(r2 * r_, y3), d5((r2 * r_) * r2, y5), d7(((r2 * r_) * r2) * r2, y5 * y2) {}
+  __device__ __forceinline__ SharedDivisors(double r2, double y)
+      : SharedDivisors(r2, sqrt_by(r2, y), y, y * y, (y * y) * y, ((y * y) * y) * (y * y)) {}
+  __device__ __forceinline__ explicit SharedDivisors(double r2)
+      : SharedDivisors(r2, rsqrt(r2)) {}
+  __device__ __forceinline__ double inv_R3() const { return d3.inv(); }
+  __device__ __forceinline__ double r(double a) const { return d1(a); }
+  __device__ __forceinline__ double R3(double a) const { return d3(a); }
+  __device__ __forceinline__ double R5(double a) const { return d5(a); }
+  __device__ __forceinline__ double R7(double a) const { return d7(a); }
 };
 
 // The same by IEEE divisions, for distances whose seventh power nears the
 // ends of the exponent range (where a residual would not be exact).
 struct PlainDivisors {
   double b1, b3, b5, b7;
-  __device__ __forceinline__ PlainDivisors(double r2, double r_) {
+  __device__ __forceinline__ explicit PlainDivisors(double r2) {
+    const double r_ = sqrt(r2);
     b1 = r_;
     b3 = r2 * r_;
     b5 = b3 * r2;
@@ -121,7 +142,7 @@ __device__ __forceinline__ void m2p64(const double2* __restrict__ mm, double xr0
                                       double& f1, double& f2, double& ep) {
   double2 m0 = __ldg(mm + 0), m1 = __ldg(mm + 1), m2 = __ldg(mm + 2),
           m3 = __ldg(mm + 3), m4 = __ldg(mm + 4);
-  const Div dv(r2, sqrt(r2));
+  const Div dv(r2);
   const double qeff = m0.x, PD0 = m0.y, PD1 = m1.x, PD2 = m1.y;
   const double PQ0 = m2.x, PQ1 = m2.y, PQ2 = m3.x, PQQ0 = m3.y, PQQ1 = m4.x,
                PQQ2 = m4.y;
@@ -166,25 +187,26 @@ __device__ __noinline__ void m2p64_extreme(const double2* __restrict__ mm, doubl
 // (pair64_far2), as leaf_pair64 evaluates them: there exp() changes no bit.
 template <int PHYS>
 __device__ __forceinline__ void leaf_pair64_far(double xr0, double xr1, double xr2, double r2,
-                                                double r, double ff, double& f0, double& f1,
-                                                double& f2, double& ep) {
-  const double y = __drcp_rn(r);
+                                                double ff, double& f0, double& f1, double& f2,
+                                                double& ep, double& r) {
+  const double y = rsqrt(r2);
+  r = sqrt_by(r2, y);
+  const Divisor dr(r, y);
   if (PHYS == 1) {
-    ep = 0.5 * ff * y;
-    const double r3 = r2 * r;
-    const double fr = div_by(ff, r3, __drcp_rn(r3));
+    ep = 0.5 * ff * dr.inv();
+    const double fr = Divisor(r2 * r, (y * y) * y)(ff);
     f0 = fr * xr0;
     f1 = fr * xr1;
     f2 = fr * xr2;
   } else {
-    const double y2 = __drcp_rn(r2);
-    ep = div_by(0.5 * ff, r, y);
+    const Divisor dr2(r2, y * y);
+    ep = dr(0.5 * ff);
     // like charges: ff x / r / r2; unlike: ff x (1/r) / r2
     const bool like = ff > 0.0;
-    const double a0 = ff * xr0, a1 = ff * xr1, a2 = ff * xr2;
-    f0 = div_by(like ? div_by(a0, r, y) : a0 * y, r2, y2);
-    f1 = div_by(like ? div_by(a1, r, y) : a1 * y, r2, y2);
-    f2 = div_by(like ? div_by(a2, r, y) : a2 * y, r2, y2);
+    const double yr = dr.inv(), a0 = ff * xr0, a1 = ff * xr1, a2 = ff * xr2;
+    f0 = dr2(like ? dr(a0) : a0 * yr);
+    f1 = dr2(like ? dr(a1) : a1 * yr);
+    f2 = dr2(like ? dr(a2) : a2 * yr);
   }
 }
 
@@ -367,8 +389,7 @@ __global__ void __launch_bounds__(kW64Threads, kW64Blocks)
                 double r = 0.0;
                 bool counted = true;
                 if (r2 > pair64_far2<PHYS>(same, tsp, wp) && r2 > 1e-72 && r2 < 1e72) {
-                  r = sqrt(r2);
-                  leaf_pair64_far<PHYS>(x0, x1, x2, r2, r, same ? kEps : -1.0 * kEps, t0, t1, t2, e);
+                  leaf_pair64_far<PHYS>(x0, x1, x2, r2, same ? kEps : -1.0 * kEps, t0, t1, t2, e, r);
                 } else {
                   const bool self = PHYS == 1 && same && __ldg(&tv.node_pt[node]) == (int)o;
                   counted = leaf_pair64<PHYS>(x0, x1, x2, r2, same, tsp, self, wp, t0, t1, t2, e, r);
