@@ -45,3 +45,13 @@ def test_colocated_noise_in_a_shared_walk(device_lib, oracle_lib):
     # the reference's own order of operations reproduces
     x = np.random.default_rng(3).standard_normal((6200, 3)) * 60.0
     _compare(x, x.copy(), 0.6, api.PHYS_REF, None)
+
+
+@pytest.mark.parametrize("side,theta", [(12, 0.5), (24, 0.5), (24, 1.0)])
+def test_ties_of_the_acceptance_test(device_lib, oracle_lib, side, theta):
+    # lattice points at powers of two: many cells lie exactly at the limit, or
+    # within rounding of it, where the squared test falls back to the root
+    g = (np.arange(side) - side // 2).astype(float)
+    x = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3) * 4.0
+    x[:] = x[np.random.default_rng(side).permutation(len(x))]
+    _compare(x[::2], x[1::2], theta, api.PHYS_REF, None)

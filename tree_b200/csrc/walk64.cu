@@ -21,14 +21,14 @@ namespace tg {
 // What bounds it: instruction issue and the latency of dependent operations at
 // 16 warps per SM (128 registers, 12 KB of shared memory a warp); the FP64 pipe
 // is busy less than half of the time, the memory side is served by L1 and L2.
-// At N = 262,144 (theta 0.5, reference laws, RDF) the walk takes 23.4 ms, half of
+// At N = 262,144 (theta 0.5, reference laws, RDF) the walk takes 21.7 ms, half of
 // it walking and summing, half evaluating: 58.9 ms with one thread per target
 // and 20 IEEE divisions per cell (16.5 of 32 lanes active), 25.2 with quotients
-// of three operations.  At N = 4,096 it takes 0.30 ms against 7.3,
+// of three operations and sums slot by slot.  At N = 4,096 it takes 0.29 ms against 7.3,
 // where a thread per target left one warp per SM.  Per SM, 12 warps (156
 // registers) and 20 (96, spills) were slower, 27.7 and 30.6 ms when 16 took 25.2;
 // so were blocks of one warp (26.2), a stack of 768 entries (26.2: fewer nodes at
-// a time near its limit).
+// a time near its limit), and children pushed a lane each by ballots (23.0 when 21.7).
 constexpr int kW64Warps = 4;
 constexpr int kW64Threads = 32 * kW64Warps;
 constexpr int kW64Blocks = 4;    // per SM
@@ -64,13 +64,18 @@ struct alignas(16) W64Smem {
   unsigned short leaf_at[kW64Ring];
 };
 
-// c.w < sqrt(r2) with the IEEE square root, which is taken only where the
-// squares are too close to tell (rounding moves each by < 1e-15).
-__device__ __forceinline__ bool mac64(double w, double r2) {
-  const double t = w * w - r2;
-  if (fabs(t) > 1e-14 * r2 && r2 > 1e-280) return t < 0.0;
-  return w < sqrt(r2);
-}
+// The acceptance test w < sqrt(r2) on squares, where rounding (each square is
+// within 1e-15) cannot change it: accepted above hi, opened below lo, and by
+// the IEEE square root in between.
+struct Mac64 {
+  double lo, hi;
+  __device__ __forceinline__ explicit Mac64(double w) {
+    const double w2 = w * w;
+    const bool tiny = w2 < 1e-280;  // squares that may have lost bits
+    hi = tiny ? 1.1e-280 : w2 * (1.0 + 2e-14);
+    lo = tiny ? 0.0 : w2 * (1.0 - 2e-14);
+  }
+};
 
 // Division by b with a reciprocal of twice the working precision, hi + lo =
 // 1/b (1 + d) with |d| < 2^-101: a hi + a lo, rounded once, is the IEEE quotient
@@ -303,11 +308,23 @@ __global__ void __launch_bounds__(kW64Threads, kW64Blocks)
             if (c.w < 0.0) {
               fin_set = set | kW64Leaf;
             } else {
+              const Mac64 mac(c.w);
+              unsigned close = 0;
 #pragma unroll
               for (int t = 0; t < T; ++t) {
                 const double x0 = sm.xt[3 * t] - c.x, x1 = sm.xt[3 * t + 1] - c.y,
                              x2 = sm.xt[3 * t + 2] - c.z;
-                if (mac64(c.w, x0 * x0 + x1 * x1 + x2 * x2)) fin_set |= 1u << t;
+                const double r2 = __fma_rn(x0, x0, __fma_rn(x1, x1, x2 * x2));
+                fin_set |= r2 > mac.hi ? 1u << t : 0u;
+                close |= r2 < mac.lo ? 0u : 1u << t;
+              }
+              close &= set & ~fin_set;
+              while (close) {
+                const int t = __ffs((int)close) - 1;
+                close &= close - 1;
+                const double x0 = sm.xt[3 * t] - c.x, x1 = sm.xt[3 * t + 1] - c.y,
+                             x2 = sm.xt[3 * t + 2] - c.z;
+                if (c.w < sqrt(x0 * x0 + x1 * x1 + x2 * x2)) fin_set |= 1u << t;
               }
               fin_set &= set;
               open_set = set & ~fin_set;
@@ -440,15 +457,18 @@ __global__ void __launch_bounds__(kW64Threads, kW64Blocks)
           const int m_at = w64_oldest(sm.m2p_at, mh, mt, done, seq, kSlots);
           const int l_at = w64_oldest(sm.leaf_at, lh, ltl, done, seq, kSlots);
           const int pend = min(m_at, l_at);
+          // whole blocks of 8 slots, so that their addresses are constants
           const double* tc = sm.term + (lane < 3 * T ? lane : 0);
           for (; done + 8 <= pend; done += 8) {
+            const double* tb = tc + 3 * T * (done & (kSlots - 1));
             double v[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = tc[3 * T * ((done + j) & (kSlots - 1))];
+            for (int j = 0; j < 8; ++j) v[j] = tb[3 * T * j];
 #pragma unroll
             for (int j = 0; j < 8; ++j) sum = sum + v[j];
           }
-          for (; done < pend; ++done) sum = sum + tc[3 * T * (done & (kSlots - 1))];
+          if (fin)
+            for (; done < pend; ++done) sum = sum + tc[3 * T * (done & (kSlots - 1))];
           __syncwarp();
           if (fin ? done == seq : seq - done <= kSlots - 32) break;
           take_leaf = fin || l_at < m_at;
