@@ -69,10 +69,10 @@ TUNE_THETAS = {2: (0.14, 0.16, 0.18, 0.20, 0.22), 3: (0.20, 0.22, 0.24, 0.26, 0.
 # learned criterion on the hexadecapole far field at theta = 0.36, eta = 3e-5
 # (worst cloud rms 5.7e-5 on 4,096 targets each, 10 steps after the 13-step
 # warm-up; the tuner's fastest order-4 pick, fixed theta = 0.39, reached
-# 1.09e-4 on one cloud at that audit), two blocks per SM (the learned build's
-# register budget).
+# 1.09e-4 on one cloud at that audit), 16 warps per SM (units of 8; the most
+# that the learned build holds).
 ENSEMBLE_TUNED = dict(theta=0.36, eta=3e-5, bucket=8, order=4, blocks_per_sm=2)
-# The fixed test's own grid (its 80-register build holds three blocks per SM).
+# The fixed test's own grid: as many warps as its build holds (20 per SM).
 ENSEMBLE_FIXED_BPS = 3
 
 

@@ -1,8 +1,8 @@
 // walk_mixed.cu -- warp-group Barnes-Hut walk in mixed precision.
 //
 // The mixed path walks ONE combined tree of both species (net-charge moments
-// about each cell's particle centroid, built bottom-up by k_net_subtrees).
-// One warp owns a target group -- a contiguous sorted range of at most 32
+// about each cell's particle centroid, net.cu).  One warp (in small clouds a
+// team of warps) owns a target group -- a contiguous sorted range of at most 32
 // particles of either species inside one cell, built by k_groups -- and
 // builds ONE interaction list for it:
 //   * group MAC: a cell is accepted when rcrit = s/theta + dx (the reference
@@ -10,12 +10,12 @@
 //     centre to the group's bounding box, so every target of the group would
 //     also accept it on its own;
 //   * accepted cells go to a shared-memory ring of far-field (M2P) entries,
-//     leaves and twigs with at most `bucket` particles go to a ring of
-//     particle (P2P) entries, other twigs push their children on a per-warp
+//     the particles of leaves and of twigs with at most `bucket` go to a list
+//     of pair (P2P) sources, other twigs push their children on a per-warp
 //     stack;
 //   * every 32 entries the warp stages them in shared memory and each lane
-//     evaluates them for its own target in FP32 (particle pairs two at a time
-//     on the packed f32x2 pipeline).
+//     evaluates them for its own target in FP32, two cells or two sources at a
+//     time on the packed f32x2 pipeline.
 // Precision: positions, the group centre and the MAC stay FP64.  Cells are
 // evaluated in FP32 relative to the group centre; particle pairs use a
 // two-float (hi + lo) split of the FP64 offsets, so a pair separation keeps
