@@ -24,13 +24,16 @@ __device__ __noinline__ void direct_near(double xr0, double xr1, double xr2, dou
   leaf_pair64<PHYS>(xr0, xr1, xr2, r2, same, tsp, self, wp, acc[0], acc[1], acc[2], acc[3], r);
 }
 
-// Bound by FP64 issue: about 28 FP64 instructions a pair, a reciprocal square
-// root among them.  The sources of a tile are taken electrons first, so that
-// charge and law are fixed inside each loop.  16,384 targets x 262,144 sources
-// of erf-Kelbg pairs: a call takes 7.5 ms, against 23.2 ms with the square
-// root and the IEEE divisions of the general law for every pair.
+// Bound by FP64 issue and its latency: about 28 FP64 instructions a pair, a
+// reciprocal square root among them.  The sources of a tile are taken electrons
+// first, so that charge and law are fixed inside each loop.  16,384 targets x
+// 262,144 sources of erf-Kelbg pairs: a call takes 6.3 ms, against 23.2 ms with
+// the square root and the IEEE divisions of the general law for every pair.
+// Registers for eight blocks per SM (64; 7.5 ms with six of 80 and 1.44 waves of
+// blocks, 8.0 with ten of 48); two sources at once needed 96 and took 7.7 ms.
+constexpr int kDirBlocks = 8;  // per SM
 template <int PHYS>
-__global__ void __launch_bounds__(kDirT)
+__global__ void __launch_bounds__(kDirT, kDirBlocks)
     k_direct(const double* __restrict__ x, int n, int n_el,
              const int64_t* __restrict__ targets, int nt, int chunk,
              WalkParams wp, double4* __restrict__ partial) {
@@ -62,7 +65,7 @@ __global__ void __launch_bounds__(kDirT)
         const double q = same ? kEps : -kEps, far2 = pair64_far2<PHYS>(same, tsp, wp);
         const int k1 = ssp ? m : me;
         double g0 = 0.0, g1 = 0.0, g2 = 0.0, e = 0.0;  // Coulomb sums of unit charges
-#pragma unroll 4
+#pragma unroll 8
         for (int k = ssp ? me : 0; k < k1; ++k) {
           const double4 s = src[k];
           const double xr0 = xt0 - s.x, xr1 = xt1 - s.y, xr2 = xt2 - s.z;
@@ -114,9 +117,14 @@ __global__ void k_direct_reduce(const double4* __restrict__ partial, int nt,
 }
 
 int direct_chunks(int n, int nt) {
-  // enough blocks to fill 148 SMs several times over
+  // All blocks take equally long, so as many as fit into whole waves of the 148
+  // SMs: one wave for few targets, whose chunks are short already (64 x 262,144:
+  // 0.28 ms, 0.31 with 1.33 waves), four above, where the part of a wave left
+  // empty by the division by the tiles is small (16,384 x 262,144: 6.4 ms,
+  // against 6.8 with two waves and 7.7 with one).
   int tiles = (nt + kDirT - 1) / kDirT;
-  int want = (8 * 148 + tiles - 1) / (tiles > 0 ? tiles : 1);
+  const int waves = tiles > 8 ? 4 : 1;
+  int want = waves * kDirBlocks * 148 / (tiles > 0 ? tiles : 1);
   int maxc = (n + kDirT - 1) / kDirT;
   if (want > maxc) want = maxc;
   return want < 1 ? 1 : want;
