@@ -24,7 +24,7 @@ __device__ __noinline__ void direct_near(double xr0, double xr1, double xr2, dou
   leaf_pair64<PHYS>(xr0, xr1, xr2, r2, same, tsp, self, wp, acc[0], acc[1], acc[2], acc[3], r);
 }
 
-// Bound by FP64 issue and its latency: about 28 FP64 instructions a pair, a
+// Bound by FP64 issue and its latency: about 19 FP64 instructions a pair, a
 // reciprocal square root among them.  The sources of a tile are taken electrons
 // first, so that charge and law are fixed inside each loop.  16,384 targets x
 // 262,144 sources of erf-Kelbg pairs: a call takes 6.3 ms, against 23.2 ms with
