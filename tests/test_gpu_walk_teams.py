@@ -93,3 +93,10 @@ def test_a_team_gives_one_warps_bits(device_lib, learned):
                 st = tf.get_state()
             np.testing.assert_array_equal(fe[ens.offsets[k]:ens.offsets[k + 1]],
                                           np.vstack([st["f_el"], st["f_ion"]]))
+
+
+@pytest.mark.parametrize("n", [15998, 16000, 29998, 30000])
+def test_teams_of_two(device_lib, n):
+    test_every_pair_once(device_lib, n // 2, n // 2)
+    for learned in (False, True):
+        test_accuracy_and_repeatability(device_lib, n, learned)

@@ -55,7 +55,7 @@ constexpr int kStackWarps = 32;   // per SM: stacks of the walk's and the sample
 template <bool RDF, bool LEARNED>
 constexpr int walk_warps() { return RDF || LEARNED ? 16 : 20; }
 
-// Warps that share a group.  Below about 20,000 particles there are fewer
+// Warps that share a group.  Below about 30,000 particles there are fewer
 // groups (of about 25 targets) than half the warps of the GPU, and a group is a
 // serial walk; a team's leader walks, and its warps evaluate the same batches
 // that one warp would, in rounds, so the forces are the same to the last bit.
@@ -65,7 +65,15 @@ constexpr int walk_warps() { return RDF || LEARNED ? 16 : 20; }
 //   N = 8,192   0.422 0.261 0.290 0.377 | 0.517 0.291 0.315 0.402
 //   N = 16,384  0.553 0.468 0.551 0.793 | 0.609 0.501 0.599 0.836
 //   N = 32,768  0.895 0.908 1.196 1.843 | 0.947 0.990 1.297 1.959
-int walk_team(int n) { return n < 3000 ? 16 : (n < 6000 ? 8 : (n < 20000 ? 4 : 1)); }
+// and for 1, 2, 4 warps, another cloud:
+//   N = 12,000  0.424 0.356 0.299 | 0.495 0.393 0.328
+//   N = 16,384  0.488 0.429 0.437 | 0.573 0.461 0.463
+//   N = 20,000  0.605 0.511 0.549 | 0.712 0.553 0.582
+//   N = 28,000  0.748 0.675 0.758 | 0.866 0.721 0.810
+//   N = 32,768  0.803 0.832 0.860 | 0.906 0.883 0.929
+int walk_team(int n) {
+  return n < 3000 ? 16 : (n < 6000 ? 8 : (n < 16000 ? 4 : (n < 30000 ? 2 : 1)));
+}
 
 constexpr int kCandRing = 64;     // power of two, > 31 + 32
 constexpr int kCellF4 = 9;        // float4 per staged far-field cell (order 4)
@@ -119,7 +127,7 @@ __device__ __forceinline__ void phi_add(WarpSmem& sm, int lane, double all, doub
 
 // A team of warps and its queue of batches: the leader walks and fills it, every
 // warp evaluates one batch a round, the leader adds the results in order.
-constexpr int kTeamMin = 4;
+constexpr int kTeamMin = 2;
 constexpr int kTeamQueue = 15 + 13;  // one short of the largest team, and what a walk's end adds
 struct TeamSmem {
   int item, take;            // the team's group; batches of this round (0: group done)
@@ -836,7 +844,7 @@ constexpr size_t walk_smem_bytes(int warps) {
   return sizeof(WarpSmem) * warps + walk_learned_bytes<LEARNED, RDF>() +
          (RDF ? sizeof(uint32_t) * 2 * kRdfBins : 0);
 }
-constexpr size_t kTeamBytes = sizeof(TeamSmem) * (16 / kTeamMin);
+constexpr size_t kTeamBytes = sizeof(TeamSmem) * (16 / kTeamMin);  // the most a launch takes
 static_assert(walk_smem_bytes<true, true>(16) + kTeamBytes <= 227 * 1024, "team walk over 227 KB");
 static_assert(walk_smem_bytes<true, true>(16) <= 195 * 1024, "RDF walk over the 196 KB step");
 static_assert(walk_smem_bytes<false, false>(20) <= 163 * 1024, "walk over the 164 KB step");
@@ -1457,7 +1465,8 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
     auto kfn = k_walk_mixed<P, R, LL, O, S>;                                  \
     const int most = S ? 16 : walk_warps<R, LL>();                            \
     const int nw = S || R || kWarpStep * bps > most ? most : kWarpStep * bps; \
-    const size_t sb = walk_smem_bytes<LL, R>(nw) + (S ? kTeamBytes : 0);      \
+    const size_t sb = walk_smem_bytes<LL, R>(nw) +                            \
+                      (S ? sizeof(TeamSmem) * (nw / a.team) : 0);             \
     static unsigned attr_set = 0; /* devices with the smem limit raised */    \
     if (dev < 32 && !(attr_set & (1u << dev))) {                              \
       cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
