@@ -248,20 +248,25 @@ __device__ __forceinline__ double warp_max_d(double v) {
 // Net monopole Q, dipole D, trace-free second moment S (from 1/2 sum q a a^T),
 // third moment T (from sum q a a a) and fourth moment H about the cell
 // centroid.  With d = target - centroid, r = |d|, s = 1/r, n = d / r:
-//   phi = s [Q + s (D.n + s (S'nn + s (T'nnn + s H'nnnn)))],
-//   -grad phi = s^2 (g n - s W),  g = r phi + 2 s n.W,
-//   W = D + 2 s (S'n + 3/2 s (T'nn + 4/3 s H'nnn)),
-// with S' = 3 S, T' = 5/2 T, H' = 35/8 H: the prefactors of each order are
-// taken into the moments when a cell is staged (once per 32 targets), and the
-// force needs no scalar of its own beyond n.W.  Normalised form: every
-// intermediate is bounded by n (a/r)^k -- escaped electrons millions of um
-// away would otherwise overflow T(d,d,d) ~ |T| r^3 while 1/r^7 underflows.
+//   r phi = Q + s D.n + 3 s^2 S(n,n) + 5/2 s^3 T(n,n,n) + 35/8 s^4 H(n,n,n,n),
+//   r^2 (-grad phi) = g n - s D - 6 s^2 S n - 15/2 s^3 T(.,n,n) - 35/2 s^4 H(.,n,n,n),
+//   g = Q + 3 s D.n + 15 s^2 S(n,n) + 35/2 s^3 T(n,n,n) + 315/8 s^4 H(n,n,n,n).
+// Normalised form: every intermediate is bounded by n (a/r)^k -- escaped
+// electrons millions of um away would otherwise overflow T(d,d,d) ~ |T| r^3
+// while 1/r^7 underflows.
 // T is trace-free (T_iik = 0), so T_kzz = -T_kxx - T_kyy and each component
 // of T(., n, n) takes five terms with a2 = nx^2 - nz^2, b2 = ny^2 - nz^2; each
 // component of H(., n, n, n) is a combination of seven cubic harmonics P1..P7
 // of n, its z component reading the dependent components xxzz, xyzz, yyzz
-// staged with the others.  About 105 multiply-adds at order 4.  The ion part
+// staged with the others.  About 120 multiply-adds at order 4.  The ion part
 // of phi for the Epot_e/Epot_i split is taken at monopole order (q_ion / r).
+//
+// The order of the operations below is part of the results: a loop of steps
+// amplifies a last-bit difference by the close passages of the electrons (ten
+// steps at N = 32,768: 1.2e-5 of the electron positions, 9e-4 of a single one).
+// The walk without RDF counts adds the cells up one after the other, the one with
+// counts in two sums, and the two form P1, P5 and P6 in different orders, as
+// their first versions did.
 
 // 1/sqrt(x) of a normal number, without rsqrtf's rescaling of subnormal ones.
 __device__ __forceinline__ float rsqrt_normal(float x) {
@@ -270,32 +275,29 @@ __device__ __forceinline__ float rsqrt_normal(float x) {
   return y;
 }
 
-// The rows of a staged cell (WarpSmem::cell), moments scaled as above.
+// The rows of a staged cell (WarpSmem::cell).
 template <int ORDER, int ROWS>
 __device__ __forceinline__ void m2p_rows(const MixedArgs& a, int node, double Gx, double Gy,
                                          double Gz, float4 (&r)[ROWS]) {
   const double4 c = ldg_d4(&a.node_c[node]);
   const float4* mp = a.mom + 3 * (int64_t)node;
-  const float4 m0 = __ldg(mp), m1 = __ldg(mp + 1), m2 = __ldg(mp + 2);
+  const float4 m0 = __ldg(mp), m2 = __ldg(mp + 2);
   r[0] = make_float4((float)(Gx - c.x), (float)(Gy - c.y), (float)(Gz - c.z), m0.x);
   r[1] = make_float4(m0.y, m0.z, m0.w, m2.w);
-  r[2] = make_float4(3.f * m1.x, 3.f * m1.y, 3.f * m1.z, 3.f * m1.w);
-  r[3] = make_float4(3.f * m2.x, 3.f * m2.y, 0.f, 0.f);
+  r[2] = __ldg(mp + 1);
+  r[3] = make_float4(m2.x, m2.y, 0.f, 0.f);
   if constexpr (ORDER >= 3) {
     const float4* tp = a.mom3 + 3 * (int64_t)node;
     const float4 t0 = __ldg(tp), t1 = __ldg(tp + 1), t2 = __ldg(tp + 2);
-    r[3].z = 2.5f * t0.x;
-    r[3].w = 2.5f * t0.y;
-    r[4] = make_float4(0.f, 2.5f * t0.w, 2.5f * t1.x, 2.5f * t1.y);
-    r[5] = make_float4(2.5f * t1.z, 2.5f * t1.w, 2.5f * t2.x, 2.5f * t2.y);
+    r[3].z = t0.x;
+    r[3].w = t0.y;
+    r[4] = make_float4(t0.z, t0.w, t1.x, t1.y);
+    r[5] = make_float4(t1.z, t1.w, t2.x, t2.y);
   }
   if constexpr (ORDER >= 4) {
     const float4* hp = a.mom4 + 3 * (int64_t)node;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float4 h = __ldg(hp + k);
-      r[6 + k] = make_float4(4.375f * h.x, 4.375f * h.y, 4.375f * h.z, 4.375f * h.w);
-    }
+    for (int k = 0; k < 3; ++k) r[6 + k] = __ldg(hp + k);
   }
 }
 
@@ -306,8 +308,25 @@ __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+// a + b that is not merged into a multiply-add with a product a or b, which
+// __fadd2_rn is.
+__device__ __forceinline__ float2 add2_apart(float2 a, float2 b) {
+  return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
 
-template <int ORDER>
+// sum += a b for the two cells of a pair: side by side, or one after the other
+// in sum.x (sum.y stays 0).
+template <bool SIDE>
+__device__ __forceinline__ void m2p_sum(float2& sum, float2 a, float2 b) {
+  if (SIDE) {
+    sum = fma2(a, b, sum);
+  } else {
+    sum.x = fmaf(a.x, b.x, sum.x);
+    sum.x = fmaf(a.y, b.y, sum.x);
+  }
+}
+
+template <int ORDER, bool RDF>
 __device__ __forceinline__ void eval_m2p(WarpSmem& sm, const int* list, int mask, int head, int cnt,
                                             const MixedArgs& a, double Gx, double Gy,
                                             double Gz, float tx, float ty, float tz,
@@ -351,12 +370,60 @@ __device__ __forceinline__ void eval_m2p(WarpSmem& sm, const int* list, int mask
     const float2 dx = add2(tx2, Ax), dy = add2(ty2, Ay), dz = add2(tz2, Az);
     const float2 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, f2(1e-30f))));
     const float2 s = make_float2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
+    const float2 s2 = mul2(s, s);
     const float2 nx = mul2(dx, s), ny = mul2(dy, s), nz = mul2(dz, s);
-    const float2 xx = mul2(nx, nx), yy = mul2(ny, ny);
-    const float2 mzz = mul2(nz, mul2(f2(-1.f), nz));
-    const float2 a2 = add2(xx, mzz), b2 = add2(yy, mzz);
-    const float2 yz2 = mul2(add2(ny, ny), nz);
-    float2 Wx = f2(0.f), Wy = Wx, Wz = Wx, ph = Wx, w = Wx;
+    q = bl[4];
+    const float2 Sxx = make_float2(q.x, q.y), Syy = make_float2(q.z, q.w);
+    q = bl[5];
+    const float2 Szz = make_float2(q.x, q.y), Sxy = make_float2(q.z, q.w);
+    q = bl[6];
+    const float2 Syz = make_float2(q.x, q.y), Szx = make_float2(q.z, q.w);
+    const float2 Sx = fma2(Sxx, nx, fma2(Sxy, ny, mul2(Szx, nz)));
+    const float2 Sy = fma2(Sxy, nx, fma2(Syy, ny, mul2(Syz, nz)));
+    const float2 Sz = fma2(Szx, nx, fma2(Syz, ny, mul2(Szz, nz)));
+    const float2 u = fma2(nx, Sx, fma2(ny, Sy, mul2(nz, Sz)));
+    q = bl[2];
+    const float2 Dx = make_float2(q.x, q.y), Dy = make_float2(q.z, q.w);
+    q = bl[3];
+    const float2 Dz = make_float2(q.x, q.y), Qi = make_float2(q.z, q.w);
+    const float2 Dn = fma2(Dx, nx, fma2(Dy, ny, mul2(Dz, nz)));
+    const float2 su = mul2(s, u);
+    float2 gp = fma2(s, fma2(f2(15.f), su, mul2(f2(3.f), Dn)), Q);
+    float2 ph = fma2(s, fma2(f2(3.f), su, Dn), Q);
+    const float2 c5 = mul2(f2(-6.f), s2), ms = mul2(f2(-1.f), s);
+    float2 gx = fma2(c5, Sx, mul2(ms, Dx));
+    float2 gy = fma2(c5, Sy, mul2(ms, Dy));
+    float2 gz = fma2(c5, Sz, mul2(ms, Dz));
+    const float2 mnz = mul2(f2(-1.f), nz);
+    if (ORDER >= 3) {
+      // (Syz Szx Txxx Tyyy) (Tzzz Txxy Txxz Txyy) (Tyyz Txzz Tyzz Txyz)
+      q = bl[7];
+      const float2 Txxx = make_float2(q.x, q.y), Tyyy = make_float2(q.z, q.w);
+      q = bl[8];
+      const float2 Txxy = make_float2(q.z, q.w);
+      q = bl[9];
+      const float2 Txxz = make_float2(q.x, q.y), Txyy = make_float2(q.z, q.w);
+      q = bl[10];
+      const float2 Tyyz = make_float2(q.x, q.y), Txzz = make_float2(q.z, q.w);
+      q = bl[11];
+      const float2 Tyzz = make_float2(q.x, q.y), Txyz = make_float2(q.z, q.w);
+      const float2 mzz = mul2(nz, mnz);
+      const float2 a2 = fma2(nx, nx, mzz), b2 = fma2(ny, ny, mzz);
+      const float2 x2 = mul2(f2(2.f), nx);
+      const float2 xy2 = mul2(x2, ny), xz2 = mul2(x2, nz), yz2 = mul2(mul2(f2(2.f), ny), nz);
+      const float2 Tx = fma2(Txxx, a2, fma2(Txyy, b2, fma2(Txxy, xy2, fma2(Txxz, xz2, mul2(Txyz, yz2)))));
+      const float2 Ty = fma2(Txxy, a2, fma2(Tyyy, b2, fma2(Txyy, xy2, fma2(Txyz, xz2, mul2(Tyyz, yz2)))));
+      const float2 Tz = fma2(Txxz, a2, fma2(Tyyz, b2, fma2(Txyz, xy2, fma2(Txzz, xz2, mul2(Tyzz, yz2)))));
+      const float2 T3 = fma2(nx, Tx, fma2(ny, Ty, mul2(nz, Tz)));
+      const float2 s3 = mul2(s2, s);
+      const float2 s3T3 = mul2(s3, T3);
+      gp = fma2(f2(17.5f), s3T3, gp);
+      ph = fma2(f2(2.5f), s3T3, ph);
+      const float2 c7 = mul2(f2(-7.5f), s3);
+      gx = fma2(c7, Tx, gx);
+      gy = fma2(c7, Ty, gy);
+      gz = fma2(c7, Tz, gz);
+    }
     if (ORDER >= 4) {
       // (xxxx xxxy xxxz xxyy) (xxyz xyyy xyyz yyyy) (yyyz xxzz xyzz yyzz)
       q = bl[12];
@@ -371,75 +438,45 @@ __device__ __forceinline__ void eval_m2p(WarpSmem& sm, const int* list, int mask
       const float2 H8 = make_float2(q.x, q.y), H9 = make_float2(q.z, q.w);
       q = bl[17];
       const float2 H10 = make_float2(q.x, q.y), H11 = make_float2(q.z, q.w);
-      const float2 x3 = mul2(f2(3.f), nx), y3 = mul2(f2(3.f), ny);
-      const float2 P1 = mul2(nx, fma2(f2(3.f), mzz, xx));
-      const float2 P6 = mul2(ny, fma2(f2(3.f), mzz, yy));
-      const float2 P2 = mul2(y3, a2), P4 = mul2(x3, b2), P5 = mul2(x3, yz2);
+      const float2 xx = mul2(nx, nx), yy = mul2(ny, ny);
+      float2 P1, P5, P6;
+      if (RDF) {
+        const float2 mzz3 = mul2(f2(-3.f), mul2(nz, nz));
+        P1 = mul2(nx, add2_apart(xx, mzz3));
+        P6 = mul2(ny, add2_apart(yy, mzz3));
+        P5 = mul2(mul2(f2(6.f), nx), mul2(ny, nz));
+      } else {
+        const float2 m3nz = mul2(f2(-3.f), nz);
+        P1 = mul2(nx, fma2(m3nz, nz, xx));
+        P6 = mul2(ny, fma2(m3nz, nz, yy));
+        P5 = mul2(mul2(mul2(f2(6.f), nx), ny), nz);
+      }
+      const float2 P2 = mul2(mul2(f2(3.f), ny), fma2(nz, mnz, xx));
+      const float2 P4 = mul2(mul2(f2(3.f), nx), fma2(nz, mnz, yy));
+      const float2 mzz = mul2(mnz, nz);
       const float2 P3 = mul2(nz, fma2(f2(3.f), xx, mzz));
       const float2 P7 = mul2(nz, fma2(f2(3.f), yy, mzz));
-      Wx = fma2(H0, P1, fma2(H1, P2, fma2(H2, P3, fma2(H3, P4,
-           fma2(H4, P5, fma2(H5, P6, mul2(H6, P7)))))));
-      Wy = fma2(H1, P1, fma2(H3, P2, fma2(H4, P3, fma2(H5, P4,
-           fma2(H6, P5, fma2(H7, P6, mul2(H8, P7)))))));
-      Wz = fma2(H2, P1, fma2(H4, P2, fma2(H9, P3, fma2(H6, P4,
-           fma2(H10, P5, fma2(H8, P6, mul2(H11, P7)))))));
-      ph = fma2(nx, Wx, fma2(ny, Wy, mul2(nz, Wz)));
-      w = ph;
+      const float2 Vx = fma2(H0, P1, fma2(H1, P2, fma2(H2, P3, fma2(H3, P4,
+                        fma2(H4, P5, fma2(H5, P6, mul2(H6, P7)))))));
+      const float2 Vy = fma2(H1, P1, fma2(H3, P2, fma2(H4, P3, fma2(H5, P4,
+                        fma2(H6, P5, fma2(H7, P6, mul2(H8, P7)))))));
+      const float2 Vz = fma2(H2, P1, fma2(H4, P2, fma2(H9, P3, fma2(H6, P4,
+                        fma2(H10, P5, fma2(H8, P6, mul2(H11, P7)))))));
+      const float2 H4n = fma2(nx, Vx, fma2(ny, Vy, mul2(nz, Vz)));
+      const float2 s4 = mul2(s2, s2);
+      const float2 s4H = mul2(s4, H4n);
+      gp = fma2(f2(39.375f), s4H, gp);
+      ph = fma2(f2(4.375f), s4H, ph);
+      const float2 c9 = mul2(f2(-17.5f), s4);
+      gx = fma2(c9, Vx, gx);
+      gy = fma2(c9, Vy, gy);
+      gz = fma2(c9, Vz, gz);
     }
-    q = bl[6];
-    const float2 Syz = make_float2(q.x, q.y), Szx = make_float2(q.z, q.w);
-    if (ORDER >= 3) {
-      // (Syz Szx Txxx Tyyy) (- Txxy Txxz Txyy) (Tyyz Txzz Tyzz Txyz)
-      q = bl[7];
-      const float2 Txxx = make_float2(q.x, q.y), Tyyy = make_float2(q.z, q.w);
-      q = bl[8];
-      const float2 Txxy = make_float2(q.z, q.w);
-      q = bl[9];
-      const float2 Txxz = make_float2(q.x, q.y), Txyy = make_float2(q.z, q.w);
-      q = bl[10];
-      const float2 Tyyz = make_float2(q.x, q.y), Txzz = make_float2(q.z, q.w);
-      q = bl[11];
-      const float2 Tyzz = make_float2(q.x, q.y), Txyz = make_float2(q.z, q.w);
-      const float2 x2 = add2(nx, nx);
-      const float2 xy2 = mul2(x2, ny), xz2 = mul2(x2, nz);
-      const float2 Tx = fma2(Txxx, a2, fma2(Txyy, b2, fma2(Txxy, xy2, fma2(Txxz, xz2, mul2(Txyz, yz2)))));
-      const float2 Ty = fma2(Txxy, a2, fma2(Tyyy, b2, fma2(Txyy, xy2, fma2(Txyz, xz2, mul2(Tyyz, yz2)))));
-      const float2 Tz = fma2(Txxz, a2, fma2(Tyyz, b2, fma2(Txyz, xy2, fma2(Txzz, xz2, mul2(Tyzz, yz2)))));
-      const float2 t = fma2(nx, Tx, fma2(ny, Ty, mul2(nz, Tz)));
-      const float2 s43 = mul2(f2(4.f / 3.f), s);
-      Wx = fma2(s43, Wx, Tx);
-      Wy = fma2(s43, Wy, Ty);
-      Wz = fma2(s43, Wz, Tz);
-      ph = fma2(s, ph, t);
-      w = fma2(s43, w, t);
-    }
-    q = bl[4];
-    const float2 Sxx = make_float2(q.x, q.y), Syy = make_float2(q.z, q.w);
-    q = bl[5];
-    const float2 Szz = make_float2(q.x, q.y), Sxy = make_float2(q.z, q.w);
-    const float2 Sx = fma2(Sxx, nx, fma2(Sxy, ny, mul2(Szx, nz)));
-    const float2 Sy = fma2(Sxy, nx, fma2(Syy, ny, mul2(Syz, nz)));
-    const float2 Sz = fma2(Szx, nx, fma2(Syz, ny, mul2(Szz, nz)));
-    const float2 u = fma2(nx, Sx, fma2(ny, Sy, mul2(nz, Sz)));
-    q = bl[2];
-    const float2 Dx = make_float2(q.x, q.y), Dy = make_float2(q.z, q.w);
-    q = bl[3];
-    const float2 Dz = make_float2(q.x, q.y), Qi = make_float2(q.z, q.w);
-    const float2 s15 = mul2(f2(1.5f), s), s2x = add2(s, s);
-    Wx = fma2(s2x, fma2(s15, Wx, Sx), Dx);
-    Wy = fma2(s2x, fma2(s15, Wy, Sy), Dy);
-    Wz = fma2(s2x, fma2(s15, Wz, Sz), Dz);
-    const float2 Dn = fma2(Dx, nx, fma2(Dy, ny, mul2(Dz, nz)));
-    ph = fma2(s, fma2(s, fma2(s, ph, u), Dn), Q);
-    w = fma2(s2x, fma2(s15, w, u), Dn);
-    const float2 s2 = mul2(s, s);
-    const float2 g = mul2(s2, fma2(s2x, w, ph));
-    const float2 ms3 = mul2(s2, mul2(f2(-1.f), s));
-    fx = fma2(g, nx, fma2(ms3, Wx, fx));
-    fy = fma2(g, ny, fma2(ms3, Wy, fy));
-    fz = fma2(g, nz, fma2(ms3, Wz, fz));
-    pa = fma2(s, ph, pa);
-    pi = fma2(Qi, s, pi);
+    m2p_sum<RDF>(fx, s2, fma2(gp, nx, gx));
+    m2p_sum<RDF>(fy, s2, fma2(gp, ny, gy));
+    m2p_sum<RDF>(fz, s2, fma2(gp, nz, gz));
+    m2p_sum<RDF>(pa, s, ph);
+    m2p_sum<RDF>(pi, Qi, s);
   }
   __syncwarp();
   out.fx = fx.x + fx.y;
@@ -994,7 +1031,7 @@ __global__ void __launch_bounds__(32 * (TEAM ? 16 : walk_warps<RDF, LEARNED>()),
     float lsum = 0.f;  // lanes 0..19: one summed coefficient of the local expansion
     bool overflow = false;
     int cqh = 0, cqt = 0;  // learned-MAC candidate ring (warp-uniform)
-    bool fin = false;
+    bool fin = false;  // the walk has ended: what is left of the lists is next
     int qn = 0;  // TEAM: batches in the queue
     while (TEAM || !fin) {
       // ---- a batch of nodes (TEAM: until a round's worth of work waits) ----
@@ -1145,7 +1182,9 @@ __global__ void __launch_bounds__(32 * (TEAM ? 16 : walk_warps<RDF, LEARNED>()),
         ssize += ktot;
         max_stack = max(max_stack, ssize);
         __syncwarp();
-        fin = ssize == 0 && cqt == cqh;
+        // remainders come after every full batch, in the order of the sums: a
+        // walk that ends on a full far-field batch takes an empty turn more
+        fin = ssize == 0 && cqt == cqh && m2t - m2h < 32;
         if (!TEAM) break;
         // full batches, and what is left once the walk has ended, to the queue
         int p2h = 0;
@@ -1219,7 +1258,7 @@ __global__ void __launch_bounds__(32 * (TEAM ? 16 : walk_warps<RDF, LEARNED>()),
       }
       while (TEAM ? kind == 1 : m2t - m2h >= 32 || (fin && m2t > m2h)) {
         if (!TEAM) cnt = min(32, m2t - m2h);
-        eval_m2p<ORDER>(sm, TEAM ? ts.idx[rank] : sm.m2p, TEAM ? 31 : kM2pRing - 1, TEAM ? 0 : m2h,
+        eval_m2p<ORDER, RDF>(sm, TEAM ? ts.idx[rank] : sm.m2p, TEAM ? 31 : kM2pRing - 1, TEAM ? 0 : m2h,
                         cnt, a, sm.gx, sm.gy, sm.gz, thx, thy, thz, lane, out);
         if (TEAM) break;
         batch_add(sm, lane, acc, out);
