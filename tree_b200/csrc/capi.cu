@@ -114,8 +114,8 @@ struct tree_gpu_handle {
   tree_gpu_timing timing{};
   std::vector<EventSet> events;
   std::string last_error;
-  // step loop: CUDA graphs of the step body, [sample][last][rdf]
-  StepGraph graphs[2][2][2];
+  // step loop: CUDA graphs of the step body, one per graph_index
+  StepGraph graphs[16];
   bool use_graphs = true;
   uint64_t epoch = 1;        // bumped whenever a captured argument may change
   bool capturing = false;    // a step body is being captured into a graph
@@ -452,11 +452,18 @@ void enqueue_step_body(tree_gpu_handle* h, double dt, bool sample, bool last,
   if (ev) record(h, ev->e[3]);
 }
 
+// The variants of enqueue_step_body: a sample step with a series buffer appends
+// a record, one without (tree_gpu_step, or no records wanted) does not.
+int graph_index(const tree_gpu_handle* h, bool sample, bool last, bool rdf) {
+  const bool append = sample && h->series;
+  return sample + 2 * last + 4 * rdf + 8 * append;
+}
+
 // The captured graph of a step-body variant, captured on first use or after
 // any argument it holds changed; nullptr when capture is not possible on
 // this stream (the caller then enqueues the body directly).
 StepGraph* graph_for(tree_gpu_handle* h, double dt, bool sample, bool last, bool rdf) {
-  StepGraph& g = h->graphs[sample][last][rdf];
+  StepGraph& g = h->graphs[graph_index(h, sample, last, rdf)];
   if (g.exec && g.epoch == h->epoch && g.dt == dt) return &g;
   if (g.exec) cudaGraphExecDestroy(g.exec);
   if (g.graph) cudaGraphDestroy(g.graph);
@@ -512,15 +519,13 @@ StepGraph* graph_for(tree_gpu_handle* h, double dt, bool sample, bool last, bool
 }
 
 void free_graphs(tree_gpu_handle* h) {
-  for (auto& a : h->graphs)
-    for (auto& b2 : a)
-      for (StepGraph& g : b2) {
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        if (g.graph) cudaGraphDestroy(g.graph);
-        if (g.has_ev)
-          for (int k = 0; k < 4; ++k) cudaEventDestroy(g.ev.e[k]);
-        g = StepGraph();
-      }
+  for (StepGraph& g : h->graphs) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (g.graph) cudaGraphDestroy(g.graph);
+    if (g.has_ev)
+      for (int k = 0; k < 4; ++k) cudaEventDestroy(g.ev.e[k]);
+    g = StepGraph();
+  }
 }
 
 // The step loop of main.f90:123-160 for nsteps steps.  Step Nloop samples
@@ -535,9 +540,7 @@ int run_impl(tree_gpu_handle* h, double dt, int32_t nsteps, int32_t nsamp,
   const tree_gpu_params& p = h->prm;
   events_for(h, (size_t)nsteps + 1);  // grow first: references below stay valid
   EventSet& et = events_for(h, 0);
-  for (auto& a : h->graphs)
-    for (auto& b2 : a)
-      for (StepGraph& g : b2) g.replays = 0;
+  for (StepGraph& g : h->graphs) g.replays = 0;
   std::vector<char> own_ev((size_t)nsteps, 0);  // step s recorded events[1 + s]
   cudaEventRecord(et.e[0], h->st);
   tg::kick_drift(h->x, h->v, h->f, n, ne, h->ion_flag, dt, p.xm_el, p.xm_ion, h->st);
@@ -591,13 +594,11 @@ int run_impl(tree_gpu_handle* h, double dt, int32_t nsteps, int32_t nsamp,
     h->timing.ms_build += elapsed(ev.e[0], ev.e[1]);
     h->timing.ms_walk += elapsed(ev.e[1], ev.e[2]);
   }
-  for (auto& a : h->graphs)
-    for (auto& b2 : a)
-      for (StepGraph& g : b2)
-        if (g.replays > 0) {
-          h->timing.ms_build += g.replays * elapsed(g.ev.e[0], g.ev.e[1]);
-          h->timing.ms_walk += g.replays * elapsed(g.ev.e[1], g.ev.e[2]);
-        }
+  for (StepGraph& g : h->graphs)
+    if (g.replays > 0) {
+      h->timing.ms_build += g.replays * elapsed(g.ev.e[0], g.ev.e[1]);
+      h->timing.ms_walk += g.replays * elapsed(g.ev.e[1], g.ev.e[2]);
+    }
   h->timing.ms_total += elapsed(et.e[0], et.e[1]);
   h->timing.calls += nsteps;
   h->nloop += nsteps;
