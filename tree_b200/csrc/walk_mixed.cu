@@ -658,7 +658,8 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, const int* list, int cnt,
                                          int p_self, int tsp, bool act, int lane,
                                          uint32_t* hist, Batch& out) {
   {
-    // this lane's source (or, past cnt, a chargeless dummy beyond any RDF bin)
+    // this lane's source (or, past cnt, a chargeless dummy: its r^2 overflows to
+    // infinity, whose inverse root is 0 and whose bin, 0 times infinity, is none)
     float v[8];
     if (lane < cnt) {
       const int s = list[lane];
@@ -669,7 +670,7 @@ __device__ __forceinline__ void eval_p2p(WarpSmem& sm, const int* list, int cnt,
       v[4] = (float)(rx - (double)hx); v[5] = (float)(ry - (double)hy);
       v[6] = (float)(rz - (double)hz); v[7] = __int_as_float(s);
     } else {
-      v[0] = v[1] = v[2] = 1.0e18f;
+      v[0] = v[1] = v[2] = 1.0e20f;
       v[3] = 0.f;
       v[4] = v[5] = v[6] = 0.f;
       v[7] = __int_as_float(-1);
