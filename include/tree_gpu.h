@@ -139,7 +139,8 @@ int tree_gpu_load_state(tree_gpu_handle* h, const double* x_el,
 /* Step drop-in for the loop body main.f90:125-131 + VVerletNotemp2: nsteps x
  * (VVerletNotemp1 -> Force -> VVerletNotemp2) on the device with no host
  * traffic.  Kinetic sums are sampled on the last step; `out` may be NULL.
- * Each step body is replayed as a CUDA graph (tree_gpu_set_graphs). */
+ * Each step body is replayed as a CUDA graph (tree_gpu_set_graphs).  An error in
+ * any of the steps is the call's (the state is then to be loaded again). */
 int tree_gpu_step(tree_gpu_handle* h, double dt, int32_t nsteps,
                   tree_gpu_diag* out);
 

@@ -25,10 +25,17 @@
 namespace tg {
 
 // ---------------------------------------------------------------- bbox ----
+// A build starts without errors; those of the builds before it (the steps of
+// one call) are kept beside them until the host has read them.
+__device__ __forceinline__ void start_errors(int32_t* err) {
+  err[1] |= err[0];
+  err[0] = 0;
+}
+
 __global__ void k_bbox_init(uint64_t* bb, int32_t* err) {
   int t = threadIdx.x;
   if (t < 12) bb[t] = (t & 1) ? 0ull : ~0ull;
-  if (t == 0) *err = 0;
+  if (t == 0) start_errors(err);
 }
 
 __device__ __forceinline__ uint64_t shfl_min_u64(uint64_t v) {
@@ -849,7 +856,10 @@ __global__ void k_topology(const key128* __restrict__ keys,
 // me, m: nodes of the first tree, of both.
 __device__ __forceinline__ void write_bounds(int me, int m, int cap, int32_t* bounds,
                                              int32_t* err) {
-  if (m > cap) set_error(err, kErrCapacity);
+  if (m > cap) {
+    set_error(err, kErrCapacity);
+    bounds[5] = m > bounds[5] ? m : bounds[5];
+  }
   bounds[0] = 0;
   bounds[1] = me < cap ? me : cap;
   bounds[2] = m < cap ? m : cap;
@@ -1125,7 +1135,7 @@ __global__ void __launch_bounds__(kFrontThreads)
 __global__ void __launch_bounds__(kFrontThreads)
     k_bbox_small(const double* __restrict__ x, int n, int n_el, Geom* g, uint64_t* bb,
                  int32_t* err) {
-  if (threadIdx.x == 0) *err = 0;
+  if (threadIdx.x == 0) start_errors(err);
   if (threadIdx.x < 12) bb[threadIdx.x] = (threadIdx.x & 1) ? 0ull : ~0ull;
   __syncthreads();
   bbox_of(x, n, n_el, threadIdx.x, blockDim.x, bb, err);

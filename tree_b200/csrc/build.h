@@ -72,8 +72,9 @@ struct BuildBuffers {
   // small
   uint64_t* bbox;       // 6 per segment (>= 2 segments)
   Geom* geom;           // per segment (>= 2)
-  int32_t* bounds;      // 5: 0, M_e, M (clamped to cap), M (untruncated), long-tie flag
-  int32_t* err;
+  int32_t* bounds;      // 6: 0, M_e, M (clamped to cap), M (untruncated), long-tie flag,
+                        // the most nodes of a build that did not fit
+  int32_t* err;         // 2: error bits of this build and its walk, of those before
   MixedNodes mx;
   Ensemble ens;
 };

@@ -4,6 +4,7 @@
 // step loop (main.f90:125-131) for one GPU: one device-resident tree per
 // species instead of the 8-rank octant decomposition and ghost-tree exchange.
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -56,8 +57,8 @@ struct StepGraph {
 // 4,096 particles took 0.474 ms (mixed) and 0.617 ms (FP64) when each result was
 // its own pageable copy; with this block and the staging below 0.346 and 0.505 ms.
 struct Status {
-  int32_t err;        // BuildBuffers::err
-  int32_t bounds[5];  // BuildBuffers::bounds
+  int32_t err[2];     // BuildBuffers::err
+  int32_t bounds[6];  // BuildBuffers::bounds
   int32_t series_count;
   int32_t pad;
   // [0..3] this step's walk counts, [4..7] running totals of the handle,
@@ -230,7 +231,7 @@ int alloc_all(tree_gpu_handle* h) {
   if ((rc = dalloc(h, &b.geom, 2))) return rc;
   if ((rc = dalloc(h, &h->status, 1))) return rc;
   b.bounds = h->status->bounds;  // addresses in device memory, not read here
-  b.err = &h->status->err;
+  b.err = h->status->err;
   h->series_count = &h->status->series_count;
   h->counters = h->status->counters;
   h->diag = h->status->diag;
@@ -346,13 +347,15 @@ void enqueue_force(tree_gpu_handle* h, bool with_rdf, EventSet* ev) {
 }
 
 // Ends a call's device work: reads the status block back, waits for the
-// stream, and turns the error word into a return code.
+// stream, and turns the errors of all its builds and walks into a return code.
 int check_device_status(tree_gpu_handle* h, bool* grow) {
   *grow = false;
   CK(cudaMemcpyAsync(h->h_pinned, h->status, sizeof(Status), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
-  const int32_t err = h->h_pinned->err;
+  const int32_t err = h->h_pinned->err[0] | h->h_pinned->err[1];
   h->timing.n_nodes = h->h_pinned->bounds[3];
+  if (err)  // reported below: the next call starts without them
+    CK(cudaMemsetAsync(h->status, 0, offsetof(Status, series_count), h->st));
   if (err & tg::kErrNonFinite)
     return fail(h, TREE_GPU_ERR_NONFINITE, "non-finite particle position");
   if (err & tg::kErrDepth)
@@ -367,7 +370,7 @@ int check_device_status(tree_gpu_handle* h, bool* grow) {
 }
 
 int grow_nodes(tree_gpu_handle* h) {
-  int need = h->h_pinned->bounds[3];
+  int need = h->h_pinned->bounds[5];
   if (need <= h->b.cap) need = h->b.cap;
   int64_t cap = (int64_t)need + need / 4 + 64;
   if (cap > 0x7fffffff) return fail(h, TREE_GPU_ERR_CAPACITY, "node count overflow");
