@@ -723,6 +723,7 @@ int tree_gpu_force(tree_gpu_handle* h, const double* x_el, const double* x_ion,
   const size_t be = 3 * sizeof(double) * (size_t)h->n_el;
   const size_t bi = 3 * sizeof(double) * (size_t)h->n_ion;
   double* stage = h->h_stage;
+  h->has_state = false;  // the device positions are this call's, not a state
   if (stage) {
     if (be) std::memcpy(stage, x_el, be);
     if (bi) std::memcpy(stage + 3 * h->n_el, x_ion, bi);
@@ -743,7 +744,6 @@ int tree_gpu_force(tree_gpu_handle* h, const double* x_el, const double* x_ion,
   }
   rc = force_device(h, with_rdf, true);
   h->has_fprev = false;
-  h->has_state = false;  // the device positions are now this call's, not a state
   if (rc) return rc;
   if (stage) {
     if (be) std::memcpy(f_el, stage, be);
