@@ -53,12 +53,12 @@ class Trial:
 
 
 def default_space(learned=True):
-    # 16 and 24 warps per SM: the learned criterion's build holds at most 16,
-    # the fixed test's 20 (more are clamped)
+    # 16 and 24 warps per SM: the fixed test's build holds at most 20 (more are
+    # clamped), the learned criterion's 16, which leaves it one choice
     thetas = (0.26, 0.28, 0.30, 0.32, 0.35)
     etas = (0.0, 1e-5, 3e-5, 1e-4) if learned else (0.0,)
     return [Candidate(t, e, b, 3, g) for t, e, b, g in
-            itertools.product(thetas, etas, (6, 8), (2, 3))]
+            itertools.product(thetas, etas, (6, 8), (2, 3)) if e == 0.0 or g == 2]
 
 
 def select(trials, target, margin=0.9):
