@@ -96,7 +96,7 @@ struct tree_gpu_handle {
   tg::MlpPacked* mlp_packed = nullptr;
   bool has_model = false;
   bool has_fprev = false;        // h->f holds forces of the current positions' predecessor
-  float mac_eta = 1e-5f, mac_rho_lo = 0.2f, mac_rho_hi = 0.9f;
+  float mac_eta = 1e-5f, mac_rho_hi = 0.9f;
   float* smp_feats = nullptr;    // collected training samples
   float* smp_labels = nullptr;
   float* smp_extra = nullptr;
@@ -267,7 +267,6 @@ tg::TreeView tree_view(tree_gpu_handle* h) {
   tg::TreeView tv;
   tv.node_c = h->b.node_c;
   tv.node_m = h->b.node_m;
-  tv.node_skip = h->b.node_skip;
   tv.node_pt = h->b.node_pt;
   tv.tree_bounds = h->b.bounds;
   return tv;
@@ -332,12 +331,11 @@ void enqueue_force(tree_gpu_handle* h, bool with_rdf, EventSet* ev) {
       lm.margins = h->mlp_stats + 64;
       lm.f_prev = h->f;  // each target's previous force, read before it is overwritten
       lm.eta = h->mac_eta;
-      lm.rho_lo = h->mac_rho_lo;
       lm.rho_hi = h->mac_rho_hi;
     }
     // the walk, and with the learned criterion its per-cell pre-filter pass
     h->timing.launches +=
-        tg::walk_mixed(h->mb, h->b, h->x, h->n, (int)h->n_el, tv, wp, h->tune,
+        tg::walk_mixed(h->mb, h->b, h->n, tv, wp, h->tune,
                        use_learned ? &lm : nullptr, h->b.ens, h->cloud_pk, h->f, h->epot_part,
                        with_rdf ? h->rdf : nullptr, h->counters, h->b.err, st);
   }
@@ -1465,7 +1463,6 @@ int tree_gpu_mac_config(tree_gpu_handle* h, float eta, float rho_lo, float rho_h
     return fail(h, TREE_GPU_ERR_ARG, "bad learned-MAC configuration");
   h->mac_eta = eta;
   ++h->epoch;
-  h->mac_rho_lo = rho_lo;
   h->mac_rho_hi = rho_hi;
   return TREE_GPU_OK;
 }

@@ -29,7 +29,6 @@ struct TreeView {
   const double4* __restrict__ node_c;  // (centre xyz, rcrit); rcrit<0: leaf
   const double2* __restrict__ node_m;  // 5 x double2 per node: qeff,D0 | D1,D2
                                        // | Q0,Q1 | Q2,QQ0 | QQ1,QQ2
-  const int32_t* __restrict__ node_skip;  // pre-order index past subtree
   const int32_t* __restrict__ node_pt;    // leaf: particle index (global)
   const int32_t* __restrict__ tree_bounds;  // [0]=0, [1]=M_e, [2]=M
 };

@@ -146,7 +146,6 @@ struct MixedArgs {
   const int32_t* __restrict__ bounds;
   const int2* __restrict__ groups;
   const int32_t* __restrict__ n_groups;
-  int n, n_el;
   int32_t* control;
   int32_t* stack;
   int team;  // warps that share a group (TEAM builds; a power of two)
@@ -156,7 +155,6 @@ struct MixedArgs {
   // loc_eps, h the group's half-diagonal, d the distance from its centre to
   // the cell's centroid; loc_eps = 0: never
   double loc_eps2;
-  int physics;
   float inv_lam2_ee, inv_lam2_ei, inv_lam2_ii;
   float inv_lam_ee, inv_lam_ei, inv_lam_ii;
   float rs_inv;
@@ -180,8 +178,6 @@ struct MixedArgs {
   const float* margins;  // m_lo, m_hi, pre-filter coefficients c0..c4
   const double* f_prev;
   float eta_over_eps;
-  float rho_lo, rho_hi;
-  float lam_ei;
   // ensemble of clouds (nseg > 0): cloud ranges, roots, pair constants
   int nseg;
   const int32_t* ens_start;
@@ -1421,14 +1417,13 @@ MixedNodes mixed_nodes(const MixedBuffers& mb) {
   return m;
 }
 
-int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
-               int n, int n_el, const TreeView& tv, const WalkParams& wp,
+int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, int n,
+               const TreeView& tv, const WalkParams& wp,
                const MixedTuning& tune, const LearnedMac* learned,
                const Ensemble& ens, const float4* cloud_pk,
                double* f, double2* epot_part,
                uint32_t* rdf, unsigned long long* counters, int32_t* err,
                cudaStream_t st) {
-  (void)x;
   if (n == 0) return 0;
   MixedArgs a;
   a.node_c = tv.node_c;
@@ -1441,8 +1436,6 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
   a.bounds = tv.tree_bounds;
   a.groups = mb.groups;
   a.n_groups = mb.control + 2;
-  a.n = n;
-  a.n_el = n_el;
   a.control = mb.control;
   a.stack = mb.stack;
   a.bucket = tune.bucket < 1 ? 1 : (tune.bucket > kMaxBucket ? kMaxBucket : tune.bucket);
@@ -1453,7 +1446,6 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
   a.p2p_max = tune.order >= 4 ? 2 : (tune.order == 3 ? 4 : 2);
   if (a.p2p_max > a.bucket) a.p2p_max = a.bucket;
   a.loc_eps2 = (double)tune.loc_eps * tune.loc_eps;
-  a.physics = wp.physics;
   a.inv_lam2_ee = (float)(1.0 / (wp.lam_ee * wp.lam_ee));
   a.inv_lam2_ei = (float)(1.0 / (wp.lam_ei * wp.lam_ei));
   a.inv_lam2_ii = (float)(1.0 / (wp.lam_ii * wp.lam_ii));
@@ -1483,9 +1475,6 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
   a.mac_k = mb.mac_k;
   a.f_prev = L ? learned->f_prev : nullptr;
   a.eta_over_eps = L ? (float)(learned->eta / kEps) : 0.f;
-  a.rho_lo = L ? learned->rho_lo : 0.f;
-  a.rho_hi = L ? learned->rho_hi : 0.f;
-  a.lam_ei = (float)wp.lam_ei;
   a.nseg = ens.nseg;
   a.ens_start = ens.start;
   a.roots = ens.roots;

@@ -57,8 +57,7 @@ struct LearnedMac {
   const float* margins = nullptr;     // device, 7: m_lo, m_hi, pre-filter c0..c4
   const double* f_prev = nullptr;     // device forces of the previous step
   float eta = 1e-5f;
-  float rho_lo = 0.2f, rho_hi = 0.9f;
-  float lam_ei = 0.f;
+  float rho_hi = 0.9f;
 };
 
 int mixed_alloc_nodes(MixedBuffers& mb, int cap);
@@ -67,8 +66,8 @@ void mixed_free(MixedBuffers& mb);
 MixedNodes mixed_nodes(const MixedBuffers& mb);
 
 // Forces on every particle from both trees.  Returns kernels launched.
-int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, const double* x,
-               int n, int n_el, const TreeView& tv, const WalkParams& wp,
+int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, int n,
+               const TreeView& tv, const WalkParams& wp,
                const MixedTuning& tune, const LearnedMac* learned,
                const Ensemble& ens, const float4* cloud_pk,
                double* f, double2* epot_part,
