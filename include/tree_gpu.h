@@ -267,8 +267,8 @@ int tree_gpu_set_stream(tree_gpu_handle* h, void* stream);
  * particles (1..8) are summed particle by particle instead of being opened;
  * `blocks_per_sm` (1..4) sets the warps per SM of the walk without RDF counts,
  * in units of 8: the walk runs one block per SM, of at most 20 warps (16 with
- * the learned criterion; larger values are clamped there; with RDF counts always
- * 16); `order` (2..4) is the
+ * the learned criterion; larger values are clamped there; with RDF counts, and
+ * below 30,000 particles, always 16); `order` (2..4) is the
  * far-field expansion order (quadrupole; octupole as well, the default 3; or
  * hexadecapole as well, 4).  A learned acceptance model predicts the error of
  * one order: load one trained at the order in use.

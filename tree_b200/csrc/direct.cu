@@ -121,7 +121,10 @@ int direct_chunks(int n, int nt) {
   // SMs: one wave for few targets, whose chunks are short already (64 x 262,144:
   // 0.28 ms, 0.31 with 1.33 waves), four above, where the part of a wave left
   // empty by the division by the tiles is small (16,384 x 262,144: 6.4 ms,
-  // against 6.8 with two waves and 7.7 with one).
+  // against 6.8 with two waves and 7.7 with one).  Chunks are then rounded up to
+  // whole tiles of sources, so few sources give fewer blocks (2,048 targets x
+  // 65,536: 3.46 waves), and tree_gpu_direct_static takes no more chunks than
+  // its fixed scratch holds (16,384 targets: 14, which is 1.51 waves).
   int tiles = (nt + kDirT - 1) / kDirT;
   const int waves = tiles > 8 ? 4 : 1;
   int want = waves * kDirBlocks * 148 / (tiles > 0 ? tiles : 1);

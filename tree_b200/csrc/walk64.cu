@@ -5,13 +5,16 @@
 // tree, then the ion tree, once for all of them: every target takes its own
 // decisions, and an entry of the walk carries the set of targets that are
 // still interested in it.  The 32 lanes test the next 32 nodes in pre-order at
-// a time and evaluate 32 (interaction, target) pairs at a time; the four sums
-// of each target (force, potential) are then taken one interaction after the
-// other in pre-order, the order of the recursive Search_Tree_ee/_ie/_ei/_ii
-// (tree.f90:721-1133).  Decisions, terms and sums are the reference's to the
-// last bit, except where the device exp() differs from the host's by an ulp:
-// an electron on its ion feels forces that cancel to rounding noise, and even
-// that noise is reproduced.
+// a time and evaluate 32 (interaction, target) pairs at a time; the three sums
+// of each target's force are then taken one interaction after the other in
+// pre-order, the order of the recursive Search_Tree_ee/_ie/_ei/_ii
+// (tree.f90:721-1133).  Decisions, terms and force sums are the reference's to
+// the last bit, except where the device exp() differs from the host's by an ulp
+// and in one quotient of 10^14 (Divisor): an electron on its ion feels forces
+// that cancel to rounding noise, and even that noise is reproduced.  The
+// potential is an FP64 sum in another order: each lane adds the terms that it
+// evaluates, then the lanes of a target are added (within 1e-12 of the gross
+// sum of the reference's).
 #include "internal.cuh"
 #include "pair64.cuh"
 #include "walk.h"
@@ -43,9 +46,11 @@ static_assert(kW64Reserve > 7 * (kMaxLevel + 1), "stack reserve");
 
 // Four targets share a walk when their warps still fill the GPU: the union of
 // their interactions is 1.2 times a single target's at N = 262,144 but is
-// walked once (25.2 ms against 43 with a target per warp).  Below about 12k
-// targets a warp per target is faster (8,192: 0.75 against 0.78 ms; 4,096:
-// 0.34 against 0.45 ms; 16,384: 1.64 against 1.45 ms).
+// walked once (21.7 ms against 36.8 with a target per warp).  A target per
+// warp | four: N = 2,048 0.127 | 0.211 ms, 4,096 0.283 | 0.358, 8,192 0.612 |
+// 0.543, 12,288 1.01 | 0.90, 16,384 1.35 | 1.09.  The line was drawn when
+// 8,192 took 0.75 | 0.78; the kernel's later steps moved the crossing to about
+// 6,000.
 constexpr int kW64Share = 12288;
 
 // Stack entries are a node and a set of targets; one whose node is accepted

@@ -44,12 +44,14 @@ constexpr int kMaxBucket = 8;
 constexpr int kP2pBuf = 31 + 32 * kMaxBucket + 1;  // what a batch of nodes can leave
 constexpr int kMaxBlocksPerSm = 4;
 // One block per SM.  The fixed test without RDF counts runs 20 warps of 96
-// registers: N = 1M takes 10.75 ms, against 11.1 ms for 16 warps of 128 and
-// 11.9 ms for 24 of 80, whose far field had to go one cell at a time and
-// spilled.  The learned criterion's build runs 16 warps of 128 (20 of 96: 1.4 %
-// slower at N = 4M, 0.6 % faster on the ensemble; 24 of 80: 7 to 24 % slower),
-// and so do the builds with RDF counts, whose histograms (2 x 10001 u32, added
-// to the global bins once, when the block ends) leave no room for more.
+// registers: N = 1M takes 11.0 ms, against 11.6 ms for 16 warps (of 96 too) and
+// 11.6 ms for 24 of 80.  The learned criterion's build runs 16 warps of 128:
+// 70.3 ms at N = 4M and 50.5 ms on the ensemble of 64 clouds.  The line was
+// drawn with a far field of fewer operations and more live registers, where
+// 20 of 96 were 1.4 % slower and 0.6 % faster; with this one they take 68.4 and
+// 49.1 ms, 24 of 80 71.6 and 50.1.  The builds with RDF counts run 16 warps:
+// their histograms (2 x 10001 u32, added to the global bins once, when the
+// block ends) leave no room for more.
 constexpr int kWarpStep = 8;      // warps per unit of the blocks_per_sm tunable
 constexpr int kStackWarps = 32;   // per SM: stacks of the walk's and the sampler's warps
 template <bool RDF, bool LEARNED>
@@ -59,18 +61,17 @@ constexpr int walk_warps() { return RDF || LEARNED ? 16 : 20; }
 // groups (of about 25 targets) than half the warps of the GPU, and a group is a
 // serial walk; a team's leader walks, and its warps evaluate the same batches
 // that one warp would, in rounds, so the forces are the same to the last bit.
-// Walk ms for 1, 4, 8, 16 warps (hexadecapole, theta 0.42, fixed | with RDF):
-//   N = 1,000   0.098 0.063 0.057 0.053 | 0.131 0.080 0.069 0.064
-//   N = 4,096   0.280 0.171 0.151 0.184 | 0.349 0.192 0.164 0.200
-//   N = 8,192   0.422 0.261 0.290 0.377 | 0.517 0.291 0.315 0.402
-//   N = 16,384  0.553 0.468 0.551 0.793 | 0.609 0.501 0.599 0.836
-//   N = 32,768  0.895 0.908 1.196 1.843 | 0.947 0.990 1.297 1.959
-// and for 1, 2, 4 warps, another cloud:
-//   N = 12,000  0.424 0.356 0.299 | 0.495 0.393 0.328
-//   N = 16,384  0.488 0.429 0.437 | 0.573 0.461 0.463
-//   N = 20,000  0.605 0.511 0.549 | 0.712 0.553 0.582
-//   N = 28,000  0.748 0.675 0.758 | 0.866 0.721 0.810
-//   N = 32,768  0.803 0.832 0.860 | 0.906 0.883 0.929
+// Walk ms for 1, 2, 4, 8, 16 warps (hexadecapole, theta 0.42, fixed | with RDF):
+//   N = 1,000   0.092 0.076 0.061 0.054 0.050 | 0.131 0.094 0.074 0.064 0.059
+//   N = 4,096   0.273 0.213 0.165 0.143 0.173 | 0.362 0.250 0.185 0.161 0.189
+//   N = 8,192   0.387 0.317 0.252 0.268 0.339 | 0.483 0.358 0.275 0.292 0.364
+//   N = 12,000  0.454 0.365 0.300 0.375 0.522 | 0.518 0.398 0.326 0.407 0.551
+//   N = 16,384  0.540 0.443 0.439 0.514 0.723 | 0.598 0.479 0.474 0.557 0.764
+//   N = 20,000  0.657 0.517 0.555 0.662 0.965 | 0.720 0.562 0.595 0.718 1.018
+//   N = 28,000  1.133 0.956 1.132 1.457 2.173 | 1.320 1.056 1.220 1.568 2.292
+//   N = 32,768  1.336 1.266 1.380 1.789 2.714 | 1.472 1.376 1.484 1.932 2.847
+// A cloud's longest groups count: on another one of 32,768 two warps took 0.832
+// against 0.803 of one, which is why the line lies below that size.
 int walk_team(int n) {
   return n < 3000 ? 16 : (n < 6000 ? 8 : (n < 16000 ? 4 : (n < 30000 ? 2 : 1)));
 }
@@ -1025,7 +1026,7 @@ __global__ void __launch_bounds__(32 * (TEAM ? 16 : walk_warps<RDF, LEARNED>()),
     int m2h = 0, m2t = 0;  // ring head/tail (warp-uniform)
     int p2n = 0, p2tot = 0;  // particle entries waiting, evaluated
     int lch = 0, lct = 0;                    // local-expansion ring
-    float lsum = 0.f;  // lanes 0..19: one summed coefficient of the local expansion
+    float lsum = 0.f;  // lanes below kLocCoef: one summed coefficient of the expansion
     bool overflow = false;
     int cqh = 0, cqt = 0;  // learned-MAC candidate ring (warp-uniform)
     bool fin = false;  // the walk has ended: what is left of the lists is next
