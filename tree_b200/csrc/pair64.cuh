@@ -83,13 +83,14 @@ __device__ __forceinline__ bool leaf_pair64(double xr0, double xr1, double xr2,
 }
 
 // Squared distance beyond which leaf_pair64's law equals q q' eps / r to
-// double precision: for REF same-species pairs the cutoff itself (closer ones
-// contribute nothing); for REF e-i pairs r > 45 rs, where exp(-r/rs) (1 + r/rs)
+// double precision: for REF same-species pairs the cutoff 0.01 (closer ones
+// contribute nothing) with a margin for a squared distance formed with fused
+// operations, since leaf_pair64 decides on the unfused one; for REF e-i pairs r > 45 rs, where exp(-r/rs) (1 + r/rs)
 // < 2e-18; for KELBG x^2 > 40 (with a margin for its rounding), the point
 // where leaf_pair64 drops the exponential too.
 template <int PHYS>
 __device__ __forceinline__ double pair64_far2(bool same, int tsp, const WalkParams& wp) {
-  if (PHYS == 0) return same ? 0.01 : 2025.0 * (wp.rs * wp.rs);
+  if (PHYS == 0) return same ? 0.01 * (1.0 + 1e-14) : 2025.0 * (wp.rs * wp.rs);
   const double lam = same ? (tsp == 0 ? wp.lam_ee : wp.lam_ii) : wp.lam_ei;
   return 40.001 * (lam * lam);
 }
