@@ -330,13 +330,14 @@ __device__ __forceinline__ void eval_m2p(WarpSmem& sm, const int* list, int mask
                                             int lane, Batch& out) {
   constexpr int kRows = ORDER >= 4 ? 9 : (ORDER == 3 ? 6 : 4);
   {
-    // this lane's cell as kRows float4 rows (see WarpSmem::cell), or a
-    // chargeless dummy far away past cnt
+    // this lane's cell as kRows float4 rows (see WarpSmem::cell), or past cnt a
+    // chargeless dummy whose r^2 overflows to infinity: its powers of 1/r are 0
+    // (at a distance that a target can lie at, they could overflow instead)
     float4 r[kRows];
     if (lane < cnt) {
       m2p_rows<ORDER>(a, list[(head + lane) & mask], Gx, Gy, Gz, r);
     } else {
-      r[0] = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f);
+      r[0] = make_float4(1.0e20f, 1.0e20f, 1.0e20f, 0.f);
 #pragma unroll
       for (int j = 1; j < kRows; ++j) r[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
