@@ -12,6 +12,7 @@
 // global gradient once per block; k_mlp_adam applies Adam to the FP32 master
 // parameters.  The operands the mma instructions read are rounded to BF16;
 // everything else is FP32 (oracle/mlp.py emulates the same roundings).
+#include <atomic>
 #include <cstdio>
 #include "internal.cuh"
 #include "mlp.cuh"
@@ -277,11 +278,13 @@ size_t mlp_grad_smem() {
 
 int mlp_grad(const float* X, const float* Y, int n, const float* params,
              float tau, float* grad, float* loss, int blocks, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
+  static std::atomic<unsigned> attr_set{0};  // devices with the smem limit raised
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 32 || !(attr_set & (1u << dev))) {
     cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)mlp_grad_smem());
-    attr = true;
+    if (dev < 32) attr_set |= 1u << dev;
   }
   if (n <= 0) return 0;
   int tiles = (n + 31) / 32;

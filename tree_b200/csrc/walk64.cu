@@ -15,6 +15,7 @@
 // potential is an FP64 sum in another order: each lane adds the terms that it
 // evaluates, then the lanes of a target are added (within 1e-12 of the gross
 // sum of the reference's).
+#include <atomic>
 #include "internal.cuh"
 #include "pair64.cuh"
 #include "walk.h"
@@ -512,7 +513,7 @@ void walk64(const double* x, int n, int n_el, const uint32_t* order,
   do {                                                                                      \
     auto kfn = k_walk64<P, R, TT>;                                                          \
     constexpr int kSmem = kW64Warps * (int)sizeof(W64Smem<TT>);                             \
-    static unsigned attr_set = 0; /* devices with the smem limit raised */                  \
+    static std::atomic<unsigned> attr_set{0}; /* devices with the smem limit raised */      \
     if (dev >= 32 || !(attr_set & (1u << dev))) {                                           \
       cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);        \
       if (dev < 32) attr_set |= 1u << dev;                                                  \

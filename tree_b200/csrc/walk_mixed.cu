@@ -29,6 +29,7 @@
 // target.  Near field: erf-Kelbg (or the reference laws) for every particle
 // pair.  With a trained model, cells the fixed test opens may be accepted by
 // the learned criterion (mac.cuh, mac_batch below).
+#include <atomic>
 #include <cstdio>
 #include "local.cuh"
 #include "mac.cuh"
@@ -1498,11 +1499,11 @@ int walk_mixed(MixedBuffers& mb, const BuildBuffers& b, int n,
     const int nw = S || R || kWarpStep * bps > most ? most : kWarpStep * bps; \
     const size_t sb = walk_smem_bytes<LL, R>(nw) +                            \
                       (S ? sizeof(TeamSmem) * (nw / a.team) : 0);             \
-    static unsigned attr_set = 0; /* devices with the smem limit raised */    \
-    if (dev < 32 && !(attr_set & (1u << dev))) {                              \
+    static std::atomic<unsigned> attr_set{0}; /* devices with the smem limit raised */ \
+    if (dev >= 32 || !(attr_set & (1u << dev))) {                             \
       cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
                            (int)(walk_smem_bytes<LL, R>(most) + (S ? kTeamBytes : 0))); \
-      attr_set |= 1u << dev;                                                  \
+      if (dev < 32) attr_set |= 1u << dev;                                    \
     }                                                                         \
     kfn<<<mb.sms, 32 * nw, sb, st>>>(a);                                      \
   } while (0)
