@@ -386,7 +386,9 @@ constexpr int kRsBins = 256;
 // mixed | FP64 path: N = 16,400 314 -> 254 | 239 -> 190, N = 65,536 341 -> 282 |
 // 265 -> 211, N = 262,144 457 -> 423 | 417 -> 375 (with k_common_levels and
 // k_owner taking in two more launches).  The rows that all blocks read grow
-// with the square of their number.
+// with the square of their number: with them at every size, without at any,
+// N = 262,144 411 | 396 and 430 | 423, N = 300,000 450 | 419 and 448 | 452,
+// N = 400,000 537 | 517 and 524 | 518, N = 1,048,576 1096 | 1150 and 920 | 988.
 constexpr int kRsRowBlocks = 128;
 
 int radix_blocks(int n) { return (n + kRsTile - 1) / kRsTile; }
