@@ -64,3 +64,31 @@ def test_mixed_walk_of_every_pair(device_lib, n_el, n_ion, physics):
     tol = 4e-6 * _gross(x)
     for a, b in zip(got[api.PREC_MIXED], got[api.PREC_FP64]):
         assert abs(a - b) <= tol
+
+
+@pytest.mark.parametrize("order", [2, 3, 4])
+@pytest.mark.parametrize("local", [0.0, 0.08])
+@pytest.mark.parametrize("n", [4000, 32000])  # a team, one warp
+def test_far_field_split(device_lib, n, local, order):
+    # A far cell's ions enter the ions' energy as one charge at the centroid of
+    # all its particles.  Its half-diagonal is below sqrt(3)/2 theta d, so at
+    # theta = 0.2 the share is within 0.173 / (1 - 0.173) = 0.21 of itself; the sum
+    # of both energies has the whole expansion (rms 1e-4 of the gross sum).
+    h = n // 2
+    c = cloud.make_cloud(n, seed=n)
+    x_el = c.x_ion + np.random.default_rng(n).standard_normal((h, 3)) * 0.3
+    x = np.vstack([x_el, c.x_ion])
+    cfg = api.Config(theta=1e-9, physics=api.PHYS_KELBG, precision=api.PREC_FP64)
+    with api.TreeForce(h, h, cfg) as tf:
+        _, _, ee64, ei64 = tf.force(x_el, c.x_ion)
+    cfg = api.Config(theta=0.2, physics=api.PHYS_KELBG, precision=api.PREC_MIXED)
+    for rdf in (False, True):
+        bins = [np.zeros(api.RDF_BINS, np.int64) for _ in range(2)] if rdf else (None, None)
+        with api.TreeForce(h, h, cfg) as tf:
+            tf.set_tuning(8, 4, order)
+            tf.set_local_expansion(local)
+            _, _, ee, ei = tf.force(x_el, c.x_ion, *bins)
+            t = tf.timings()
+        assert t.n_m2p > 0 and (t.n_local > 0) == (local > 0)
+        assert abs(ei - ei64) <= 0.21 * _gross(c.x_ion)
+        assert abs(ee + ei - ee64 - ei64) <= 1e-4 * _gross(x)
